@@ -141,6 +141,45 @@ struct Gen {
 
   std::string T(Node *n) const { return dt_ctype(n->meta.dtype); }
 
+  // 64-bit integer nodes (cell indices and sums, differences and products of them
+  // and of scalar constants) whose value fits 32 bits on this raster: their low 32
+  // bits are the value, so the generated code computes them in 32 bits (one
+  // multiply instead of four, 32-bit conversions to float). The index bound is a
+  // size class, not the raster's size, so sources stay shared between rasters.
+  std::set<Node *> narrow;
+  void find_narrow() {
+    const double most = std::max(g.W, g.H) <= 32768 ? 32767.0 : 2147483647.0;
+    std::map<Node *, std::pair<double, double>> range;
+    auto of = [&](Node *p, double &lo, double &hi) {
+      if (literal.count(p) && !dt_is_float(p->meta.dtype)) {
+        lo = hi = var_as_f64(p->cnst);
+        return true;
+      }
+      auto it = range.find(p);
+      if (it == range.end()) return false;
+      lo = it->second.first;
+      hi = it->second.second;
+      return true;
+    };
+    for (Node *n : g.nodes) {
+      if (n->kind == K_INDEX) range[n] = {0.0, most};
+      if (n->kind != K_BINARY || n->meta.dtype != S64 || (n->op != ADD && n->op != SUB && n->op != MUL)) continue;
+      double al, ah, bl, bh;
+      if (!of(n->prev[0], al, ah) || !of(n->prev[1], bl, bh)) continue;
+      double lo, hi;
+      if (n->op == ADD) { lo = al + bl; hi = ah + bh; }
+      else if (n->op == SUB) { lo = al - bh; hi = ah - bl; }
+      else {
+        lo = std::min(std::min(al * bl, al * bh), std::min(ah * bl, ah * bh));
+        hi = std::max(std::max(al * bl, al * bh), std::max(ah * bl, ah * bh));
+        if (n->prev[0] == n->prev[1]) lo = std::max(lo, 0.0);
+      }
+      if (lo < -2147483648.0 || hi > 2147483647.0) continue;
+      range[n] = {lo, hi};
+      narrow.insert(n);
+    }
+  }
+
   // Nodes whose value is always 0 or 1: relational and logical results.
   static bool zero_one(const Node *p) {
     if (p->kind == K_BINARY) return p->op >= EQ && p->op <= OR;
@@ -483,6 +522,7 @@ struct Gen {
         }
       }
     }
+    find_narrow();
     if (Runtime::get().algebraic_rewrite && (g.skeleton == SK_LOCAL || g.skeleton == SK_FOCAL)) find_shades();
   }
 
@@ -1162,7 +1202,9 @@ struct Gen {
             if (!dt_is_float(n->prev[0]->meta.dtype) && zero_one(n->prev[0])) l = "(" + l + " ? (" + pts + ")1 : (" + pts + ")0)";
             if (!dt_is_float(n->prev[1]->meta.dtype) && zero_one(n->prev[1])) r = "(" + r + " ? (" + pts + ")1 : (" + pts + ")0)";
           }
-          s << "const " << t << " " << v << " = (" << t << ")(" << l << " " << sym << " " << r << ");";
+          // a 64-bit value that provably fits 32 bits is computed in 32
+          s << "const " << t << " " << v << " = (" << t << ")" << (narrow.count(n) ? "(s32)" : "") << "(" << l << " " << sym
+            << " " << r << ");";
         } else {
           std::string L = "(" + pts + ")(" + l + ")", R = "(" + pts + ")(" + r + ")";
           switch (n->op) {
@@ -1948,6 +1990,72 @@ static std::string gen_zonal(Gen &G) {
 // this CTA one step earlier; cells on an octant boundary are written by both
 // adjacent octants with identical values. Local nodes before the scan produce
 // `in` per cell; those after it run right after the cell's scan value.
+// The tiled form of a radial scan: an octant's triangle of (front, cell) pairs is
+// cut into strips of RADIAL_T fronts and tiles of RADIAL_B cells. A tile is one CTA's
+// work item:
+//   1. all threads evaluate the scan's argument and the interpolation weight of
+//      the tile's cells (and of the RADIAL_T cells left of it that its own cells
+//      depend on: a cell reads the previous front at d1 and d1 - 1) into shared
+//      memory, along x whichever way the octant runs;
+//   2. warp 0 takes the last front of the previous strip from the scratch area,
+//      sweeps the strip's fronts in registers, neighbours by shuffles, no
+//      barrier between fronts, and publishes its last front;
+//   3. all threads evaluate the nodes after the scan and store the outputs.
+// Tiles are claimed by ticket in strip order, so the tiles a claimed tile waits
+// for are held by CTAs already running: the wait (bounded) needs no co-residency
+// of the grid. Step 1 does not depend on the previous strip and runs before the
+// wait. Every operation is the one of the front-by-front form, so results are
+// the same bits.
+static std::string radial_tiles_source(Gen &G, const std::string &T) {
+  KernelPlan &P = G.plan;
+  Node *scan = P.core;
+  const std::string v = G.val(scan);
+  const std::string arg = G.val(scan->prev[0]), AT = G.T(scan->prev[0]);
+  P.smem_bytes = radial_tile_smem(scan->meta.dtype);
+  std::ostringstream s;
+  // the scan's argument at one cell, and the nodes after the scan
+  s << "__device__ __forceinline__ " << T << " radial_arg(const Args &a, const In &in, int x, int y) {\n" << G.center_loads(true);
+  for (Node *n : G.g.nodes) {
+    if (n == scan) break;
+    s << "    " << G.stmt(n, false) << "\n";
+  }
+  s << "    return (" << T << ")(" << arg << ");\n}\n"
+    << "__device__ __forceinline__ void radial_post(const Args &a, const In &in, int x, int y, " << T << " fin) {\n"
+    << G.center_loads(true);
+  for (Node *n : G.g.nodes) {
+    if (n == scan) s << "    const " << T << " " << v << " = fin;\n";
+    else s << "    " << G.stmt(n, false) << "\n";
+  }
+  for (auto &kv : G.outk) {
+    // a scan only this group reads is not kept: its raster is null
+    if (kv.first == scan) s << "    if (a.out[" << kv.second << "].p) ";
+    else s << "    ";
+    s << "str<" << G.T(kv.first) << ">(a.out[" << kv.second << "], x, y, " << G.val(kv.first) << ");\n";
+  }
+  s << "}\n"
+    << "typedef " << T << " RT;\n"
+    << "struct RadialOps {\n"
+    << "  typedef In Cell;\n"
+    << "  static __device__ __forceinline__ void load(const Args &a, In &in, int x, int y) { radial_load(a, in, x, y); }\n"
+    << "  static __device__ __forceinline__ RT arg(const Args &a, const In &in, int x, int y) { return radial_arg(a, in, x, y); }\n"
+    << "  static __device__ __forceinline__ RT fold(RT lit, RT v) { return is_finite(v) ? RedOp<" << scan->op
+    << ", RT>::f(lit, v) : lit; }\n"
+    << "  static __device__ __forceinline__ RT neutral() { return " << var_literal(reduction_neutral(scan->op, scan->meta.dtype))
+    << "; }\n"
+    << "  static __device__ __forceinline__ void post(const Args &a, const In &in, int x, int y, RT v) { radial_post(a, in, x, y, v); }\n"
+    << "};\n"
+    << "extern \"C\" __global__ void __launch_bounds__(RADIAL_NT, 12) KNAME_tiles(const __grid_constant__ Args a) {\n"
+    << "  radial_tiles<RadialOps, RT, RADIAL_B, RADIAL_T>(a, (int)blockIdx.x);\n"
+    << "}\n"
+    << "struct TilesManyArgs { u64 args; s64 n, per; };\n"
+    << "extern \"C\" __global__ void __launch_bounds__(RADIAL_NT, 12) KNAME_tiles_many(const __grid_constant__ TilesManyArgs m) {\n"
+    << "  const int r = (int)(blockIdx.x / m.per);\n"
+    << "  if (r >= m.n) return;\n"
+    << "  radial_tiles<RadialOps, RT, RADIAL_B, RADIAL_T>(((const Args *)m.args)[r], (int)(blockIdx.x - r * m.per));\n"
+    << "}\n";
+  return s.str();
+}
+
 static std::string gen_radial(Gen &G) {
   KernelPlan &P = G.plan;
   Node *scan = P.core;
@@ -2121,14 +2229,10 @@ static std::string gen_radial(Gen &G) {
     << "extern \"C\" __global__ void __launch_bounds__(512) KNAME_cl(const __grid_constant__ Args a) {\n"
     << "  radial_run_cluster(a, (int)(blockIdx.x / cl_size()));\n"
     << "}\n";
-  // one scan: 8 CTAs (one per octant); many scans: 8 CTAs per Args of a device array
+  s << radial_tiles_source(G, T);
+  // 8 CTAs, one per octant
   s << "extern \"C\" __global__ void __launch_bounds__(512) KNAME(const __grid_constant__ Args a) {\n"
     << "  radial_run(a, blockIdx.x);\n"
-    << "}\n"
-    << "struct ManyArgs { u64 args; s64 n; };\n"
-    << "extern \"C\" __global__ void __launch_bounds__(512) KNAME_many(const __grid_constant__ ManyArgs m) {\n"
-    << "  if ((s64)(blockIdx.x >> 3) >= m.n) return;\n"
-    << "  radial_run(((const Args *)m.args)[blockIdx.x >> 3], blockIdx.x & 7);\n"
     << "}\n";
   return s.str();
 }

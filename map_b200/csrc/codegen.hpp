@@ -101,6 +101,15 @@ const FocalTune &focal_tune();
 // Dynamic shared memory of a radial scan launch over a W x H raster: two front
 // buffers when they fit (0 otherwise: the kernel then re-reads fronts from its output).
 size_t radial_front_smem(int W, int H, int dtype);
+// The tiled form of a radial scan: own cells, fronts and threads per tile
+// (skeleton/scan.cuh RADIAL_B, RADIAL_T, RADIAL_NT), its dynamic shared memory, and
+// the scratch of a scan over a W x H raster from
+// (sx, sy) with at most `lim` fronts (lim < 0: all): bytes, zero at the start, and
+// the number of tiles.
+constexpr int kRadialB = 32, kRadialT = 32, kRadialThreads = 64;
+size_t radial_tile_smem(int dtype);
+struct RadialScratch { size_t bytes = 0; long long tiles = 0; };
+RadialScratch radial_tile_scratch(int W, int H, int sx, int sy, long long lim, int dtype);
 // Pointer-jumping flow accumulation (integer types): cell limit, rounds for N
 // cells, whether a type qualifies, and the scratch bytes for N cells.
 size_t spread_pj_cells();

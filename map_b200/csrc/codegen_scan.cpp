@@ -1,13 +1,21 @@
 // Execution of the Radiating (radial scan) and Spreading (flow accumulation)
 // skeletons; their kernels are generated in codegen.cpp (gen_radial, gen_spread).
 //
-// Radiating (runtime/skeleton/RadiatingSkeleton.cpp:32-323): one CTA per octant
-// sweeps the octant's fronts d0 = 1, 2, ... in order; the cells of a front are
-// independent and are spread over the CTA's threads. A cell's scan value is
-// op(LIT(prev front at d1, prev front at d1-1), in) when `in` is finite; the
-// start cell holds the neutral value. The previous and current fronts are kept in
-// the CTA's shared memory when both fit (radial_front_smem, up to 200 KiB); for
-// rasters at least kRadialClusterDim cells across, the octant runs on a cluster of
+// Radiating (runtime/skeleton/RadiatingSkeleton.cpp:32-323): a cell's scan value is
+// op(LIT(prev front at d1, prev front at d1-1), in) when `in` is finite; the start
+// cell holds the neutral value. The octants are cut into tiles of fronts and cells
+// that CTAs claim in strip order (codegen.cpp radial_tiles_source,
+// skeleton/scan.cuh radial_tiles): the chain of a strip's fronts runs in one warp's
+// registers, everything else of a cell beside it, and a strip waits only for the
+// last front of the one above. 4096^2 viewshed: 217 us, against 4161 us for one
+// front at a time with a cluster barrier between fronts; 8 B per cell would take 21
+// us of HBM: the 2250 fronts' chain (about 65 ns each with the exchange between
+// strips) and the issue of two IEEE divisions and square roots per cell bound it.
+// A tile reads cells that its neighbours write, so a raster evaluated into the
+// memory of one of its inputs is swept front by front instead: one CTA per octant,
+// a front's cells spread over the CTA's threads, the previous and current fronts in
+// shared memory when both fit (radial_front_smem, up to 200 KiB); for rasters at
+// least kRadialClusterDim cells across, the octant runs on a cluster of
 // kRadialCluster CTAs, each holding one segment of both fronts in its shared
 // memory and reading the value left of its segment from its neighbour's
 // (distributed shared memory). Fronts too long for either are read back from the
@@ -79,28 +87,90 @@ size_t radial_front_smem(int W, int H, int dtype) {
   return b <= (size_t)200 * 1024 ? b : 0;                          // larger: fronts re-read from the output
 }
 
+// Whether an output of the group shares memory with one of its inputs (a caller
+// may evaluate a raster into its own buffer).
+static bool overlap(const Group &g, const KernelPlan &P, std::unordered_map<Node *, DevRaster> &bufs,
+                    const std::function<DevRaster &(Node *)> &get) {
+  for (Node *o : P.out_rasters) {
+    const DevRaster &d = bufs.at(o);
+    const uintptr_t d0 = (uintptr_t)d.ptr, d1 = d0 + (uintptr_t)(d.pitch * g.H);
+    for (Node *in : P.in_rasters) {
+      const DevRaster &r = get(in);
+      const uintptr_t r0 = (uintptr_t)r.ptr, r1 = r0 + (uintptr_t)(r.pitch * g.H);
+      if (d0 < r1 && r0 < d1) return true;
+    }
+  }
+  return false;
+}
+
+size_t radial_tile_smem(int dtype) {
+  // the arguments of a tile's fronts, rows padded by four cells
+  return (size_t)kRadialT * (kRadialB + kRadialT + 4) * dt_size(dtype);
+}
+RadialScratch radial_tile_scratch(int W, int H, int sx, int sy, long long lim, int dtype) {
+  constexpr int b = kRadialB, t = kRadialT;
+  // the octants' extents along and across their axis: each pair of a side in x and a side in y twice
+  const int ex[2] = {sx, W - 1 - sx}, ey[2] = {sy, H - 1 - sy};
+  RadialScratch R;
+  size_t slots = 0;
+  auto octant = [&](int ep, int eq) {
+    const int dmax = lim >= 0 && lim < ep ? (int)lim : ep;
+    const int strips = (dmax + t - 1) / t;
+    slots += (size_t)strips * (eq / b + 1);
+    for (int s = 0; s < strips; s++) R.tiles += std::min(std::min(s * t + t, dmax), eq) / b + 1;
+  };
+  for (int i = 0; i < 2; i++)
+    for (int j = 0; j < 2; j++) {
+      octant(ex[i], ey[j]);
+      octant(ey[j], ex[i]);
+    }
+  R.bytes = 64 + slots * b * 2 * dt_size(dtype);
+  return R;
+}
+
 void run_scan_group(const Group &g, const KernelPlan &P, std::unordered_map<Node *, DevRaster> &bufs,
                     const std::function<DevRaster &(Node *)> &get, const std::function<DevRaster(Node *)> &alloc_out) {
   CudaEnv &env = CudaEnv::get();
   cudaStream_t st = (cudaStream_t)env.stream();
-  for (Node *o : P.out_rasters)
-    if (!bufs.count(o)) bufs[o] = alloc_out(o);
   Node *scan = P.core;
-  KernelHandle kh = env.kernel(P.source, P.kname, 0);
+  for (Node *o : P.out_rasters) {
+    if (bufs.count(o)) continue;
+    if (o == scan && g.scan_private && scan->kind == K_RADIALSCAN) {
+      DevRaster none;   // the tiled form keeps no raster that only the group itself reads
+      none.dtype = o->meta.dtype;
+      none.W = g.W;
+      none.H = g.H;
+      bufs[o] = none;
+    } else {
+      bufs[o] = alloc_out(o);
+    }
+  }
   if (scan->kind == K_RADIALSCAN) {
-    int ri = -1;
-    for (size_t k = 0; k < P.out_rasters.size(); k++)
-      if (P.out_rasters[k] == scan) ri = (int)k;
-    if (ri < 0) throw MapError("radial scan output missing");
+    const bool tiled = !overlap(g, P, bufs, get);
+    if (!tiled && !bufs.at(scan).ptr) bufs[scan] = alloc_out(scan);
     long long lim = -1;
     if (scan->radius > 0) {
       lim = (long long)scan->radius;
       for (Node *o : P.out_rasters) {
         DevRaster &r = bufs.at(o);
-        cuda_check(cudaMemset2DAsync(r.ptr, r.pitch, 0xFF, (size_t)r.W * dt_size(r.dtype), r.H, st), "memset");
+        if (r.ptr) cuda_check(cudaMemset2DAsync(r.ptr, r.pitch, 0xFF, (size_t)r.W * dt_size(r.dtype), r.H, st), "memset");
       }
     }
-    uint64_t aux[4] = {(uint64_t)scan->coord.arr[0], (uint64_t)scan->coord.arr[1], (uint64_t)lim, (uint64_t)ri};
+    uint64_t aux[4] = {(uint64_t)scan->coord.arr[0], (uint64_t)scan->coord.arr[1], (uint64_t)lim, 0};
+    if (tiled) {
+      const RadialScratch R = radial_tile_scratch(g.W, g.H, scan->coord.arr[0], scan->coord.arr[1], lim, scan->meta.dtype);
+      void *work = nullptr;
+      cuda_check(cudaMallocAsync(&work, R.bytes, st), "cudaMallocAsync(radial work)");
+      cuda_check(cudaMemsetAsync(work, 0, R.bytes, st), "memset");
+      KernelHandle kt = env.kernel(P.source, P.kname + "_tiles", P.smem_bytes);
+      const long long cap = (long long)env.sm_count() * std::max(1, env.occupancy(kt, kRadialThreads, P.smem_bytes));
+      aux[3] = (uint64_t)(uintptr_t)work;
+      auto at = pack_args(g, P, get, bufs, 0, 0, g.W, g.H, aux);
+      env.launch(kt, (int)std::max<long long>(1, std::min(cap, R.tiles)), kRadialThreads, P.smem_bytes, (CUstream_st *)st, at.data(),
+                 at.size());
+      cuda_check(cudaFreeAsync(work, st), "cudaFreeAsync");
+      return;
+    }
     auto a = pack_args(g, P, get, bufs, 0, 0, g.W, g.H, aux);
     // long fronts: a cluster of kRadialCluster CTAs per octant, each holding a
     // segment of the fronts in shared memory
@@ -116,6 +186,7 @@ void run_scan_group(const Group &g, const KernelPlan &P, std::unordered_map<Node
     env.launch(env.kernel(P.source, P.kname, smem), 8, 512, smem, (CUstream_st *)st, a.data(), a.size());
     return;
   }
+  KernelHandle kh = env.kernel(P.source, P.kname, 0);
   const size_t N = (size_t)g.W * g.H;
   if (N >= (size_t)1 << 31) throw MapError("spreadScan: raster too large");
   if (N > kSpreadKahnCells && N <= spread_pj_cells() && spread_pj_type(scan->meta.dtype)) {

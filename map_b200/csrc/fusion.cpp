@@ -290,12 +290,15 @@ FusionResult fuse(const std::vector<Node *> &order, const std::set<Node *> &targ
     std::unordered_set<Node *> members(g.nodes.begin(), g.nodes.end());
     for (Node *n : g.nodes) {
       if (is_free_raster(n) && !materialise.count(n)) continue;
-      bool out = targets.count(n) > 0 || n->kind == K_RADIALSCAN || n->kind == K_SPREADSCAN ||
-                 (n->meta.numdim == D0 && n->kind == K_ZONALREDUC);
+      bool out = targets.count(n) > 0 || (n->meta.numdim == D0 && n->kind == K_ZONALREDUC);
       for (Node *c : n->next) {
         if (!in_order.count(c)) continue;
         if (c->kind == K_WRITE) out = true;
         else if (!members.count(c)) out = true;
+      }
+      if (n->kind == K_RADIALSCAN || n->kind == K_SPREADSCAN) {
+        g.scan_private = !out;
+        out = true;
       }
       if (out) g.outputs.push_back(n);
     }

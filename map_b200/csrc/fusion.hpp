@@ -35,6 +35,7 @@ struct Group {
   std::vector<Node *> nodes;    // nodes computed by the group, in id order (includes inlined FREE nodes)
   std::vector<Node *> inputs;   // rasters and scalars read from outside, in id order
   std::vector<Node *> outputs;  // nodes whose values leave the group, in id order
+  bool scan_private = false;    // the scan is among the outputs only for the sweep's own use
   std::vector<Group *> prev, next;
   // geometry shared by every raster node of the group
   int W = 0, H = 0, BS0 = 0, BS1 = 0;

@@ -40,6 +40,8 @@ long long pitch_for(int W, int dt) {
 
 // Launch phases of a batch, in stream order. A request is complete once the
 // last phase its program uses has finished.
+// CTAs that share the tiles of one request's radial scan
+constexpr long long kRadialCtas = 32;
 enum Phase { PH_LEVEL0 = 0, PH_RADIAL = 1, PH_LEVEL1 = 2, PH_SPREAD = 3, N_PHASES = 4 };
 
 struct Req {
@@ -222,7 +224,7 @@ Template &Server::Impl::template_for(int type, int w, int h, bool compile) {
       k = register_kind(P);
       T->last_phase = std::max(T->last_phase, lv == 0 ? (int)PH_LEVEL0 : (int)PH_LEVEL1);
     } else if (g.skeleton == SK_RADIAL) {
-      env.kernel(P.source, P.kname + "_many", 0);
+      env.kernel(P.source, P.kname + "_tiles_many", P.smem_bytes);
       T->last_phase = std::max(T->last_phase, (int)PH_RADIAL);
     } else if (g.skeleton == SK_SPREAD) {
       env.kernel(P.source, P.kname + "_prep_many", 0);
@@ -271,7 +273,7 @@ void Server::Impl::run_batch(std::vector<Req *> &batch) {
     const KernelPlan *plan = nullptr;
     std::vector<unsigned char> args;
     int n = 0;
-    int max_dim = 0;   // largest window side (radial front buffers)
+    long long tiles = 0;   // most tiles of a radial scan
     size_t max_cells = 0;
     bool pj = false;   // flow accumulation by pointer jumping (integer type, windows above 64 K cells)
   };
@@ -332,6 +334,10 @@ void Server::Impl::run_batch(std::vector<Req *> &batch) {
           t.dtype = o->meta.dtype;
           t.W = o->meta.W();
           t.H = o->meta.H();
+          if (g.skeleton == SK_RADIAL && o == P.core && g.scan_private) {
+            bufs[o] = t;   // read by its own group only: not kept
+            continue;
+          }
           t.pitch = pitch_for(t.W, t.dtype);
           cuda_check(cudaMallocAsync(&t.ptr, (size_t)t.pitch * t.H, st), "cudaMallocAsync(intermediate)");
           r->scratch.push_back(t.ptr);
@@ -353,19 +359,22 @@ void Server::Impl::run_batch(std::vector<Req *> &batch) {
           Many &mn = radial[P.source];
           mn.plan = &P;
           const long long lim = r->radius > 0 ? (long long)r->radius : -1;
-          int ri = 0;
-          for (size_t k = 0; k < P.out_rasters.size(); k++)
-            if (P.out_rasters[k] == P.core) ri = (int)k;
           if (lim >= 0)
             for (Node *o : P.out_rasters) {
               DevRaster &d = bufs.at(o);
+              if (!d.ptr) continue;
               cuda_check(cudaMemset2DAsync(d.ptr, d.pitch, 0xFF, (size_t)d.W * dt_size(d.dtype), d.H, st), "memset");
             }
-          uint64_t aux[4] = {(uint64_t)r->ox, (uint64_t)r->oy, (uint64_t)lim, (uint64_t)ri};
+          const RadialScratch R = radial_tile_scratch(g.W, g.H, r->ox, r->oy, lim, P.core->meta.dtype);
+          void *work = nullptr;
+          cuda_check(cudaMallocAsync(&work, R.bytes, st), "cudaMallocAsync(radial work)");
+          r->scratch.push_back(work);
+          cuda_check(cudaMemsetAsync(work, 0, R.bytes, st), "memset");
+          uint64_t aux[4] = {(uint64_t)r->ox, (uint64_t)r->oy, (uint64_t)lim, (uint64_t)(uintptr_t)work};
           auto a = pack_args(g, P, get, bufs, 0, 0, g.W, g.H, aux, &scal);
           mn.args.insert(mn.args.end(), a.begin(), a.end());
           mn.n++;
-          mn.max_dim = std::max(mn.max_dim, std::max(g.W, g.H));
+          mn.tiles = std::max(mn.tiles, R.tiles);
         } else {   // SK_SPREAD
           const size_t N = (size_t)g.W * g.H;
           const bool pj = serve_pj() && N > ((size_t)1 << 16) && spread_pj_type(P.core->meta.dtype);
@@ -466,10 +475,10 @@ void Server::Impl::run_batch(std::vector<Req *> &batch) {
   cuda_check(cudaEventRecord(ev[PH_LEVEL0], st), "cudaEventRecord");
   for (auto &kv : radial) {
     Many &mn = kv.second;
-    const size_t smem = radial_front_smem(mn.max_dim, mn.max_dim, mn.plan->core->meta.dtype);
-    KernelHandle kh = env.kernel(mn.plan->source, mn.plan->kname + "_many", smem);
-    struct { uint64_t args; int64_t n; } ma{(uint64_t)(uintptr_t)dptr[bi++], mn.n};
-    env.launch(kh, 8 * mn.n, 512, smem, (CUstream_st *)st, &ma, sizeof ma);
+    KernelHandle kh = env.kernel(mn.plan->source, mn.plan->kname + "_tiles_many", mn.plan->smem_bytes);
+    const int64_t per = std::max<long long>(1, std::min<long long>(mn.tiles, kRadialCtas));
+    struct { uint64_t args; int64_t n, per; } ma{(uint64_t)(uintptr_t)dptr[bi++], mn.n, per};
+    env.launch(kh, (int)(mn.n * per), kRadialThreads, mn.plan->smem_bytes, (CUstream_st *)st, &ma, sizeof ma);
   }
   cuda_check(cudaEventRecord(ev[PH_RADIAL], st), "cudaEventRecord");
   launch_level(1);
