@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <map>
+#include <mutex>
 #include <set>
 #include <sstream>
 
@@ -966,6 +967,58 @@ struct Gen {
       if (!q_type(n->meta.dtype, r) || r.lo < 0 || r.hi > 0x7FFF) return false;
       qr[n] = r;
     }
+    return true;
+  }
+
+  // The rule of a group that maps every 3 x 3 window of zeros and ones to zero or
+  // one by its centre cell and the count of the other eight: bit n of born /
+  // survive is the next cell for n neighbours around a zero / a one. The windows
+  // are evaluated with the host's operator tables, in the kernel's order.
+  bool binary_rule(uint32_t &born, uint32_t &survive) {
+    if (plan.in_rasters.size() != 1 || plan.out_rasters.size() != 1 || staged.size() != 1 || plan.halo_x > 1 || plan.halo_y > 1 ||
+        plan.out_rasters[0]->meta.dtype != U8 || !plan.scalars.empty() || !quadable())
+      return false;
+    uint32_t seen[2] = {0, 0}, to[2] = {0, 0};
+    std::vector<Variant> v(g.nodes.size());
+    for (int window = 0; window < 512; window++) {
+      auto tap = [&](int dx, int dy) { return var_make_f64((window >> ((dy + 1) * 3 + dx + 1)) & 1, U8); };
+      auto of = [&](Node *p) {
+        auto m = member.find(p);
+        if (m != member.end()) return v[m->second];
+        if (literal.count(p)) return p->cnst;
+        return tap(0, 0);
+      };
+      for (size_t i = 0; i < g.nodes.size(); i++) {
+        Node *n = g.nodes[i];
+        const int dt = n->meta.dtype;
+        switch (n->kind) {
+          case K_CONSTANT: v[i] = var_convert(reference_literal_value(n->cnst), dt); break;
+          case K_CAST: case K_BARRIER: v[i] = var_convert(of(n->prev[0]), dt); break;
+          case K_UNARY: v[i] = var_convert(host_unary(n->op, of(n->prev[0])), dt); break;
+          case K_BINARY: v[i] = var_convert(host_binary(n->op, of(n->prev[0]), of(n->prev[1])), dt); break;
+          case K_CONDITIONAL: v[i] = var_convert(of(n->prev[var_as_f64(of(n->prev[0])) != 0.0 ? 1 : 2]), dt); break;
+          case K_NEIGHBOR: v[i] = tap(n->coord.arr[0], n->coord.arr[1]); break;
+          case K_CONVOLUTION: {
+            const int hx = n->halo_x(), hy = n->halo_y(), mw = n->mask_ds.arr[0];
+            Variant acc = var_make_f64(0.0, dt);
+            for (int i1 = -hy; i1 <= hy; i1++)
+              for (int i0 = -hx; i0 <= hx; i0++)
+                acc = var_convert(host_binary(ADD, acc, host_binary(MUL, tap(i0, i1), n->mask[(i1 + hy) * mw + (i0 + hx)])), dt);
+            v[i] = acc;
+            break;
+          }
+          default: return false;
+        }
+      }
+      const double next = var_as_f64(v[member.at(plan.out_rasters[0])]);
+      const int c = (window >> 4) & 1, n = __builtin_popcount(window & ~16);
+      if (next != 0.0 && next != 1.0) return false;
+      if ((seen[c] >> n & 1) && (to[c] >> n & 1) != (uint32_t)next) return false;
+      seen[c] |= 1u << n;
+      to[c] |= (uint32_t)next << n;
+    }
+    born = to[0];
+    survive = to[1];
     return true;
   }
 
@@ -2735,6 +2788,63 @@ bool focal_quad_form(const Group &g) {
 bool tile_cfg_valid(const TileCfg &c) {
   return c.tw > 0 && c.th > 0 && c.nt >= 32 && c.nt <= 1024 && c.nt % 32 == 0 && c.nt % c.tw == 0 &&
          (c.tw * c.th) % c.nt == 0 && c.tw <= c.nt && c.tw <= 224 && c.th <= 224;
+}
+
+bool generate_rule(const Group &g, const std::string &kname, KernelPlan &P) {
+  if (g.skeleton != SK_FOCAL || !Runtime::get().paired_cells) return false;
+  P = KernelPlan();
+  P.skeleton = SK_FOCAL;
+  Gen G(g, P);
+  G.classify();
+  // what a group's windows say depends on its generated code alone (masks and
+  // constants are in it), so every kernel is looked at once
+  struct Known { bool rule; uint32_t born, survive; };
+  static std::mutex m;
+  static std::map<std::string, Known> known;
+  Known k{false, 0, 0};
+  {
+    std::lock_guard<std::mutex> lk(m);
+    auto it = known.find(kname);
+    if (it == known.end()) {
+      k.rule = G.binary_rule(k.born, k.survive);
+      if (known.size() >= 4096) known.clear();
+      known[kname] = k;
+    } else {
+      k = it->second;
+    }
+  }
+  if (!k.rule) return false;
+  const uint32_t born = k.born, survive = k.survive;
+  std::ostringstream s;
+  s << "#include \"map_rule.cuh\"\n" << G.args_struct(0, false)
+    << "struct Rule {\n"
+    << "  static __device__ __forceinline__ u32 next(u32 s0, u32 s1, u32 s2, u32 s3, u32 c) {\n"
+    << "    u32 r = 0u;\n";
+  for (int n = 0; n <= 8; n++) {
+    const bool b = born >> n & 1, k = survive >> n & 1;
+    if (!b && !k) continue;
+    s << "    r |= ";
+    for (int i = 0; i < 4; i++) s << (n >> i & 1 ? "s" : "~s") << i << " & ";
+    s << (b && k ? "0xffffffffu" : b ? "~c" : "c") << ";\n";
+  }
+  s << "    return r;\n  }\n"
+    << "  template <class F0> static __device__ __forceinline__ u8 cell(const Args &a, const F0 &f0, int x, int y) {\n"
+    << "    const int lx = 0, ly = 0;\n"
+    << G.center_loads(false) << G.body(false) << "    return (u8)(" << G.val(P.out_rasters[0]) << ");\n  }\n};\n";
+  for (int small = 0; small < 2; small++)
+    s << "extern \"C\" __global__ void __launch_bounds__(" << kRuleThreads << ") KNAME_gens" << (small ? "_s" : "")
+      << "(const __grid_constant__ Args a) {\n"
+      << "  griddep_wait();\n"
+      << "  rule_tile<Rule, " << (small ? kRuleRowsSmall : kRuleRows) / (kRuleThreads / 32) << ", " << kRuleThreads / 32
+      << ">(a);\n}\n";
+  std::string src = s.str();
+  P.kname = "map_rule_" + fnv_hex(src).substr(0, 12);
+  size_t pos;
+  while ((pos = src.find("KNAME")) != std::string::npos) src.replace(pos, 5, P.kname);
+  P.source = src;
+  P.threads = kRuleThreads;
+  P.smem_bytes = 2 * 288 * 160;   // RULE_SMEM
+  return true;
 }
 
 KernelPlan generate_kernel(const Group &g, TileCfg cfg) {

@@ -73,6 +73,16 @@ struct KernelPlan {
 
 KernelPlan generate_kernel(const Group &g, TileCfg cfg = TileCfg());
 
+// Chained generations of a binary neighbourhood rule (skeleton/rule.cuh): the plan
+// of a kernel that runs several generations of focal group g per launch. False when
+// g is no such rule: one byte raster in and out, a window of at most 3 x 3, integer
+// nodes of the packed byte form, and every window of zeros and ones mapped to zero
+// or one by its centre cell and the count of its eight neighbours.
+bool generate_rule(const Group &g, const std::string &kname, KernelPlan &P);   // kname: g's own focal kernel
+// Columns, rows and generations of a tile of the rule kernels (KNAME_gens: 192
+// rows, KNAME_gens_s: 64, of which a row per generation is lost at both ends).
+constexpr int kRuleCols = 992, kRuleRows = 192, kRuleRowsSmall = 64, kRuleThreads = 512, kRuleMaxGens = 16, kRuleMaxGensSmall = 12;
+
 // Tuning overrides of the standalone Local / Focal skeletons, read once from the
 // environment variable MAP_B200_FOCAL_TUNE ("key=value,..."; the keys are the
 // field names below; absent = the built-in choice, which the measured defaults

@@ -398,8 +398,47 @@ Executor::Prepared Executor::prepare(const std::vector<Node *> &targets, const s
       jobs.push_back(std::async(std::launch::async, [src]() { CudaEnv::get().compile(*src); }));
     }
   }
+  find_chains(P, tset);
+  if (compile)
+    for (auto &c : P.chains)
+      if (seen.insert(c.plan.source).second) {
+        const std::string *src = &c.plan.source;
+        jobs.push_back(std::async(std::launch::async, [src]() { CudaEnv::get().compile(*src); }));
+      }
   for (auto &f : jobs) f.get();
   return P;
+}
+
+// Chains of focal groups that are generations of one binary rule (generate_rule):
+// equal kernels, each reading the previous one's only output, which nothing else
+// needs.
+void Executor::find_chains(Prepared &P, const std::set<Node *> &tset) {
+  const size_t n = P.fr.groups.size();
+  P.chain_of.assign(n, -1);
+  if (Runtime::get().exec_mode != EXEC_FUSED) return;
+  std::set<Node *> in_order(P.order.begin(), P.order.end());
+  // the group that alone consumes g's only output, if it is the same kernel
+  auto next_of = [&](const Group &g) -> const Group * {
+    const KernelPlan &K = P.plans[g.id];
+    if (g.skeleton != SK_FOCAL || K.out_rasters.size() != 1 || K.in_rasters.size() != 1 || g.next.size() != 1) return nullptr;
+    const Group &h = *g.next[0];
+    const KernelPlan &L = P.plans[h.id];
+    Node *o = K.out_rasters[0];
+    if (h.skeleton != SK_FOCAL || L.kname != K.kname || L.in_rasters.size() != 1 || L.in_rasters[0] != o || tset.count(o) ||
+        h.W != g.W || h.H != g.H || h.BS0 != g.BS0 || h.BS1 != g.BS1)
+      return nullptr;
+    for (Node *c : o->next)
+      if (in_order.count(c) && c->kind == K_WRITE) return nullptr;
+    return &h;
+  };
+  for (auto &gp : P.fr.groups) {
+    if (P.chain_of[gp->id] >= 0) continue;
+    Prepared::Chain c;
+    for (const Group *g = gp.get(); g; g = next_of(*g)) c.groups.push_back(g->id);
+    if (c.groups.size() < 2 || !generate_rule(*gp, P.plans[gp->id].kname, c.plan)) continue;
+    for (int id : c.groups) P.chain_of[id] = (int)P.chains.size();
+    P.chains.push_back(std::move(c));
+  }
 }
 
 std::shared_ptr<Executor::Prepared> Executor::prepare_cached(const std::vector<Node *> &targets,
@@ -790,6 +829,50 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
   if (rt.prediction)
     for (auto &gp : P.fr.groups)
       predicted[gp->id] = predict_group(*gp, P.plans[gp->id], fixed, rt.border) ? 1 : 0;
+  // a chain runs when none of its groups is predicted
+  std::vector<char> chained(P.chains.size(), 1);
+  for (size_t c = 0; c < P.chains.size(); c++)
+    for (int id : P.chains[c].groups)
+      if (predicted[id]) chained[c] = 0;
+  auto run_chain = [&](const Prepared::Chain &c) {
+    const Group &g = *P.fr.groups[c.groups.front()];
+    const KernelPlan &first = P.plans[g.id], &last_plan = P.plans[c.groups.back()];
+    Node *in = first.in_rasters[0], *out = last_plan.out_rasters[0];
+    const DevRaster src = get(in);
+    if (!bufs.count(out)) bufs[out] = alloc_out(out);
+    const DevRaster dst = bufs.at(out);
+    int left = (int)c.groups.size();
+    // 16 generations of a 192-row tile cost it a sixth of its rows; rasters that give
+    // fewer such tiles than half the SMs take tiles of 64 rows and 12 generations.
+    const int tx = (g.W + kRuleCols - 1) / kRuleCols;
+    auto tiles = [&](int rows, int k) { return (long long)tx * ((g.H + rows - 2 * k - 1) / (rows - 2 * k)); };
+    const bool small = tiles(kRuleRows, kRuleMaxGens) * 2 < env.sm_count();
+    const int rows = small ? kRuleRowsSmall : kRuleRows, most = small ? kRuleMaxGensSmall : kRuleMaxGens;
+    // a launch reads its neighbours' input cells: none writes what it reads
+    const uintptr_t s0 = (uintptr_t)src.ptr, d0 = (uintptr_t)dst.ptr;
+    const bool same = s0 < d0 + (uintptr_t)(dst.pitch * g.H) && d0 < s0 + (uintptr_t)(src.pitch * g.H);
+    int launches = std::max((left + most - 1) / most, same ? 2 : 1);
+    KernelHandle kh = env.kernel(c.plan.source, c.plan.kname + (small ? "_gens_s" : "_gens"), c.plan.smem_bytes);
+    std::unordered_map<Node *, DevRaster> io;
+    std::function<DevRaster &(Node *)> bound = [&](Node *n) -> DevRaster & { return io.at(n); };
+    DevRaster tmp[2], cur = src;
+    for (int i = 0; launches > 0; i++, launches--) {
+      const int k = (left + launches - 1) / launches;
+      left -= k;
+      if (launches > 1 && !tmp[i & 1].ptr) tmp[i & 1] = alloc_raster(U8, g.W, g.H);
+      io[c.plan.in_rasters[0]] = cur;
+      io[c.plan.out_rasters[0]] = cur = launches > 1 ? tmp[i & 1] : dst;
+      const uint64_t aux[4] = {(uint64_t)k, 0, 0, 0};
+      auto a = pack_args(g, c.plan, bound, io, 0, 0, g.W, g.H, aux);
+      const int ty = (g.H + rows - 2 * k - 1) / (rows - 2 * k);
+      if (rt.dependent_launch)
+        env.launch_pdl(kh, tx, ty, kRuleThreads, c.plan.smem_bytes, (CUstream_st *)st, a.data());
+      else
+        env.launch_2d(kh, tx, ty, kRuleThreads, c.plan.smem_bytes, (CUstream_st *)st, a.data());
+    }
+    for (const DevRaster &r : tmp)
+      if (r.ptr) cuda_check(cudaFreeAsync(r.ptr, st), "cudaFreeAsync");
+  };
   auto fill_predicted = [&](const Group &g, const KernelPlan &K) {
     ensure_outputs(g, K);
     for (Node *o : K.out_rasters) {
@@ -809,6 +892,11 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
         const KernelPlan &K = P.plans[g.id];
         if (g.skeleton == SK_HOST) { run_host(g); continue; }
         if (predicted[g.id]) { fill_predicted(g, K); continue; }
+        if (P.chain_of[g.id] >= 0 && chained[P.chain_of[g.id]]) {
+          const Prepared::Chain &c = P.chains[P.chain_of[g.id]];
+          if (c.groups.back() == g.id) run_chain(c);
+          continue;
+        }
         if (g.skeleton == SK_RADIAL || g.skeleton == SK_SPREAD) {
           run_scan_group(g, K, bufs, get, alloc_out);
           continue;

@@ -118,8 +118,17 @@ class Executor {
     FusionResult fr;
     std::vector<KernelPlan> plans;
     std::vector<Node *> order;
+    // Chains of groups that are generations of one binary rule, each group's output
+    // read by the next one only: run several generations per launch.
+    struct Chain {
+      std::vector<int> groups;   // group ids, in order
+      KernelPlan plan;
+    };
+    std::vector<Chain> chains;
+    std::vector<int> chain_of;   // per group: its chain, or -1
   };
   Prepared prepare(const std::vector<Node *> &targets, const std::set<Node *> &tset, bool compile);
+  static void find_chains(Prepared &P, const std::set<Node *> &tset);
   // Programs evaluated again (same target nodes, same launch mode, same known
   // scalar values, no node destroyed since) reuse their fusion and kernel plans.
   struct CacheEntry {
