@@ -1267,6 +1267,8 @@ struct Gen {
               const char *fn = n->op == ATAN2 ? "atan2" : n->op == POW ? "pow" : n->op == HYPOT ? "hypot" : "fmod";
               if (n->op == ATAN2 && pt == F32)   // map_common.cuh's atan2 (<= 1.5 ulp, about half the instructions)
                 s << "const " << t << " " << v << " = map_atan2f(" << L << ", " << R << ");";
+              else if (n->op == POW && pt == F32)    // squares and cubes by products (map_common.cuh)
+                s << "const " << t << " " << v << " = map_powf(" << L << ", " << R << ");";
               else if (dt_is_float(pt)) s << "const " << t << " " << v << " = " << float_fn(pt, fn) << "(" << L << ", " << R << ");";
               else s << "const " << t << " " << v << " = (" << t << ")" << fn << "((double)" << L << ", (double)" << R << ");";
               break;
@@ -1986,28 +1988,96 @@ static std::string gen_zonal(Gen &G) {
     if (n->kind == K_ZONALREDUC) P.zonal.push_back(n);
   const int nz = (int)P.zonal.size();
   // cell: updates the accumulators
-  s << "__device__ __forceinline__ void zonal_cell(const Args &a, int x, int y";
+  s << "struct In {\n";
+  for (Node *p : P.in_rasters) s << "  " << G.T(p) << " i" << G.rin.at(p) << ";\n";
+  s << "  int dummy;\n};\n";
+  s << "__device__ __forceinline__ void zonal_cell(const Args &a, const In &in, int x, int y";
   for (int z = 0; z < nz; z++) s << ", " << G.T(P.zonal[z]) << " &acc" << z;
-  s << ") {\n" << G.center_loads(false) << G.body(true) << G.stores() << "}\n";
+  s << ") {\n" << G.center_loads(true) << G.body(true) << G.stores() << "}\n";
+  // Full tiles of rasters of one element size es, rows on 16-byte boundaries, no
+  // raster outputs: a thread loads V = 16 / es cells of a row at a time, all of its
+  // tile's vectors first, and folds them into `sets` accumulators of each reduction
+  // in turn (shorter chains of dependent additions, and of roundings). Other tiles
+  // take one cell at a time. stats.py's seven reductions of an 8192^2 raster: 4-byte
+  // loads and one accumulator left the loads waiting on each other.
+  int es = 0;
+  bool vec = G.outk.empty() && !P.in_rasters.empty();
+  for (Node *p : P.in_rasters) {
+    const int b = (int)dt_size(p->meta.dtype);
+    if (es && b != es) vec = false;
+    es = b;
+  }
+  const int V = es ? 16 / es : 0, TV = V ? TW / V : 0;
+  if (!V || TW % V || NT % TV || TH % (NT / TV)) vec = false;
+  const int RV = vec ? TH / (NT / TV) : 0, sets = vec ? std::min(V, nz > 3 ? 2 : 4) : 1;
+  auto acc_of = [](int z, int j) { return "acc" + std::to_string(z) + (j ? "_" + std::to_string(j) : ""); };
   // main kernel: tiles strided over the grid, per-thread accumulation, CTA reduction, one partial per CTA.
   // aux[0] = partials (Scalar8[slot * nz + z]), aux[1] = first slot of this launch
   s << "extern \"C\" __global__ void __launch_bounds__(" << NT << ") KNAME(const __grid_constant__ Args a) {\n"
     << "  __shared__ Scalar8 scratch[" << NT / 32 << "];\n";
   for (int z = 0; z < nz; z++) {
     Node *n = P.zonal[z];
-    s << "  " << G.T(n) << " acc" << z << " = " << var_literal(reduction_neutral(n->op, n->meta.dtype)) << ";\n";
+    for (int j = 0; j < sets; j++)
+      s << "  " << G.T(n) << " " << acc_of(z, j) << " = " << var_literal(reduction_neutral(n->op, n->meta.dtype)) << ";\n";
   }
-  s << "  const int lx = threadIdx.x % " << TW << ", ly0 = threadIdx.x / " << TW << ";\n"
+  // the tiles blockIdx.x, blockIdx.x + gridDim.x, ...: their coordinates by steps
+  s << "  int tx = (int)blockIdx.x % a.g.tiles_x, ty = (int)blockIdx.x / a.g.tiles_x;\n"
+    << "  const int sx = (int)gridDim.x % a.g.tiles_x, sy = (int)gridDim.x / a.g.tiles_x;\n"
     << "  for (int ti = blockIdx.x; ti < a.g.tiles; ti += gridDim.x) {\n"
-    << "    const Tile t = tile_of<" << TW << ", " << TH << ">(a.g, ti);\n"
-    << "    const int x = t.x0 + lx;\n"
+    << "    const Tile t = tile_at<" << TW << ", " << TH << ">(a.g, tx, ty);\n"
+    << "    tx += sx;\n    ty += sy;\n"
+    << "    if (tx >= a.g.tiles_x) {\n      tx -= a.g.tiles_x;\n      ++ty;\n    }\n";
+  auto accs = [&](int j) {
+    std::string r;
+    for (int z = 0; z < nz; z++) r += ", " + acc_of(z, j);
+    return r;
+  };
+  if (vec) {
+    s << "    if (t.xe - t.x0 == " << TW << " && t.ye - t.y0 == " << TH << " && (((t.x0 * " << es << ")";
+    for (size_t k = 0; k < P.in_rasters.size(); k++) s << " | a.in[" << k << "].p | a.in[" << k << "].pitch";
+    s << ") & 15) == 0) {\n"
+      << "      const int x = t.x0 + (threadIdx.x % " << TV << ") * " << V << ", y0 = t.y0 + threadIdx.x / " << TV << ";\n";
+    for (Node *p : P.in_rasters) s << "      uint4 w" << G.rin.at(p) << "[" << RV << "];\n";
+    s << "#pragma unroll\n"
+      << "      for (int r = 0; r < " << RV << "; ++r) {\n";
+    for (Node *p : P.in_rasters) {
+      const int k = G.rin.at(p);
+      s << "        w" << k << "[r] = __ldg((const uint4 *)(row_ptr<" << G.T(p) << ">(a.in[" << k << "], y0 + r * " << NT / TV
+        << ") + x));\n";
+    }
+    s << "      }\n"
+      << "#pragma unroll\n"
+      << "      for (int r = 0; r < " << RV << "; ++r) {\n"
+      << "        In in;\n";
+    for (int j = 0; j < V; j++) {
+      for (Node *p : P.in_rasters) {
+        const int k = G.rin.at(p);
+        s << "        in.i" << k << " = vlane<" << G.T(p) << ">(w" << k << "[r], " << j << ");\n";
+      }
+      s << "        zonal_cell(a, in, x + " << j << ", y0 + r * " << NT / TV << accs(j % sets) << ");\n";
+    }
+    s << "      }\n"
+      << "      continue;\n"
+      << "    }\n";
+  }
+  s << "    const int x = t.x0 + threadIdx.x % " << TW << ", ly0 = threadIdx.x / " << TW << ";\n"
     << "#pragma unroll 4\n"
     << "    for (int k = 0; k < " << TH * TW / NT << "; ++k) {\n"
     << "      const int y = t.y0 + ly0 + k * " << NT / TW << ";\n"
-    << "      if (x < t.xe && y < t.ye) zonal_cell(a, x, y";
-  for (int z = 0; z < nz; z++) s << ", acc" << z;
-  s << ");\n    }\n  }\n"
-    << "  Scalar8 *part = (Scalar8 *)a.aux[0];\n"
+    << "      if (x < t.xe && y < t.ye) {\n"
+    << "        In in;\n";
+  for (Node *p : P.in_rasters) {
+    const int k = G.rin.at(p);
+    s << "        in.i" << k << " = ldr<" << G.T(p) << ">(a.in[" << k << "], x, y);\n";
+  }
+  s << "        zonal_cell(a, in, x, y" << accs(0) << ");\n"
+    << "      }\n    }\n  }\n";
+  for (int z = 0; z < nz; z++) {
+    Node *n = P.zonal[z];
+    for (int j = 1; j < sets; j++)
+      s << "  " << acc_of(z, 0) << " = RedOp<" << n->op << ", " << G.T(n) << ">::f(" << acc_of(z, 0) << ", " << acc_of(z, j) << ");\n";
+  }
+  s << "  Scalar8 *part = (Scalar8 *)a.aux[0];\n"
     << "  const u64 slot = a.aux[1] + blockIdx.x;\n";
   for (int z = 0; z < nz; z++) {
     Node *n = P.zonal[z];
@@ -2015,7 +2085,7 @@ static std::string gen_zonal(Gen &G) {
       << "    if (threadIdx.x == 0) put_scalar<" << G.T(n) << ">(&part[slot * " << nz << " + " << z << "], r); }\n";
   }
   s << "}\n";
-  // finalisation: one CTA folds every partial in slot order, deterministically
+  // finalisation: one CTA per reduction folds its partials in slot order, deterministically
   s << "struct FinalArgs { u64 part; s64 nslots; u64 res; u64 pad; };\n";
   P.final_args_size = 32;
   s << "extern \"C\" __global__ void __launch_bounds__(" << NT << ") KNAME_final(const __grid_constant__ FinalArgs f) {\n"
@@ -2025,7 +2095,7 @@ static std::string gen_zonal(Gen &G) {
   for (int z = 0; z < nz; z++) {
     Node *n = P.zonal[z];
     std::string t = G.T(n);
-    s << "  { " << t << " acc = " << var_literal(reduction_neutral(n->op, n->meta.dtype)) << ";\n"
+    s << "  if (blockIdx.x == " << z << ") { " << t << " acc = " << var_literal(reduction_neutral(n->op, n->meta.dtype)) << ";\n"
       << "    for (s64 i = threadIdx.x; i < f.nslots; i += blockDim.x) acc = RedOp<" << n->op << ", " << t
       << ">::f(acc, get_scalar<" << t << ">(part[i * " << nz << " + " << z << "]));\n"
       << "    const " << t << " r = block_reduce<" << n->op << ", " << t << ">(acc, scratch);\n"

@@ -597,9 +597,11 @@ std::vector<PlainJob> Executor::schedule_for(const std::vector<Node *> &targets)
 void Executor::sync() {
   CudaEnv &env = CudaEnv::get();
   if (!env.device_ready()) return;
-  cuda_check(cudaStreamSynchronize((cudaStream_t)env.stream()), "stream synchronize");
+  // the read of the error word follows the stream's work: one wait for both
   uint32_t err = 0;
-  cuda_check(cudaMemcpy(&err, env.err_word(), sizeof err, cudaMemcpyDeviceToHost), "error word read");
+  cuda_check(cudaMemcpyAsync(&err, env.err_word(), sizeof err, cudaMemcpyDeviceToHost, (cudaStream_t)env.stream()),
+             "error word read");
+  cuda_check(cudaStreamSynchronize((cudaStream_t)env.stream()), "stream synchronize");
   if (err) {
     cuda_check(cudaMemset(env.err_word(), 0, sizeof err), "error word reset");
     std::string m = "device kernel reported an error:";
@@ -752,7 +754,8 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
     if (g.skeleton == SK_ZONAL) {
       ZonalState &z = zst[g.id];
       const int nz = (int)K.zonal.size();
-      const int grid = std::min(tiles, env.sm_count() * 8);
+      // one resident wave: a second, partial one would leave SMs idle
+      const int grid = std::min(tiles, env.sm_count() * std::min(8, std::max(1, env.occupancy(kh, K.threads, K.smem_bytes))));
       if (z.slots + grid > z.cap) throw MapError("zonal partial storage overflow");
       auto a = build_args(g, K, rx0, ry0, rx1, ry1, (uint64_t)(uintptr_t)z.part, (uint64_t)z.slots);
       env.launch(kh, grid, K.threads, K.smem_bytes, (CUstream_st *)st, a.data(), a.size());
@@ -799,7 +802,7 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
     KernelHandle kf = env.kernel(K.source, K.kname_final, 0);
     struct { uint64_t part; int64_t nslots; uint64_t res; uint64_t pad; } fa{(uint64_t)(uintptr_t)z.part, z.slots,
                                                                               (uint64_t)(uintptr_t)z.res, 0};
-    env.launch(kf, 1, K.threads, 0, (CUstream_st *)st, &fa, sizeof fa);
+    env.launch(kf, nz, K.threads, 0, (CUstream_st *)st, &fa, sizeof fa);
     std::vector<uint64_t> res(nz);
     cuda_check(cudaMemcpyAsync(res.data(), z.res, (size_t)nz * 8, cudaMemcpyDeviceToHost, st), "result read-back");
     cuda_check(cudaStreamSynchronize(st), "stream synchronize");

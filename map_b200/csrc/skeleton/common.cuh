@@ -136,6 +136,24 @@ template <class T> __device__ __forceinline__ void vset(uint4 &v, int j, T x) {
   memcpy((char *)&v + j * sizeof(T), &x, sizeof(T));
 }
 
+// ------------------------------------------------------------------ powers (float)
+
+// x to the power y: the square is one product, correctly rounded; the cube adds the
+// rounding errors of its two products, each exact as a fused multiply-add (Dekker,
+// Numer. Math. 18, 1971), to their result: 0.51 ulp at most, 5 instructions. Below
+// 2^-33, where those errors would underflow, the cube is taken in double. Other
+// exponents take CUDA's powf. With a literal exponent only one case is compiled.
+__device__ __forceinline__ float map_cube(float x) {
+  const float h = x * x, r = h * x;
+  const float e = __fmaf_rn(__fmaf_rn(x, x, -h), x, __fmaf_rn(h, x, -r));
+  return fabsf(r) < __int_as_float(0x7f800000) && fabsf(r) > 0.0f ? r + e : r;
+}
+__device__ __forceinline__ float map_powf(float x, float y) {
+  if (y == 2.0f) return x * x;
+  if (y == 3.0f) return fabsf(x) < 0x1p-33f ? (float)((double)x * (double)x * (double)x) : map_cube(x);
+  return powf(x, y);
+}
+
 // ------------------------------------------------------------------ atan2 (float)
 
 // Two-argument arctangent of float32 operands, at most 1.5 ulp from the
@@ -413,8 +431,11 @@ MAP_PR_F1(roundf)
   __device__ __forceinline__ PR<float> pr_##fn(const PR<float> &x, const PR<float> &y) { \
     return PR<float>(fn(x.a, y.a), fn(x.b, y.b));                                       \
   }
-MAP_PR_F2(powf) MAP_PR_F2(hypotf) MAP_PR_F2(fmodf) MAP_PR_F2(atan2f)
+MAP_PR_F2(hypotf) MAP_PR_F2(fmodf) MAP_PR_F2(atan2f)
 #undef MAP_PR_F2
+__device__ __forceinline__ PR<float> pr_powf(const PR<float> &x, const PR<float> &y) {
+  return PR<float>(map_powf(x.a, y.a), map_powf(x.b, y.b));
+}
 
 // the engine's own atan2, sin and cos on pairs: the same operations as the
 // scalar forms above (bit-identical lanes), the polynomials packed
