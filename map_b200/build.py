@@ -26,7 +26,8 @@ NVCC = os.path.join(CUDA, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 # name under which each header is visible to NVRTC-compiled kernels
-HEADERS = [("common.cuh", "map_common.cuh"), ("scan.cuh", "map_scan.cuh"), ("rule.cuh", "map_rule.cuh")]
+HEADERS = [("common.cuh", "map_common.cuh"), ("scan.cuh", "map_scan.cuh"), ("rule.cuh", "map_rule.cuh"),
+           ("flow.cuh", "map_flow.cuh")]
 
 
 def _run(cmd):

@@ -2374,7 +2374,7 @@ static std::string gen_spread(Gen &G) {
   if (!G.rin.count(scan->prev[1])) throw MapError("spreadScan: the direction raster must be materialised");
   const std::string T = G.T(scan);
   std::ostringstream s;
-  s << "#include \"map_scan.cuh\"\n" << G.args_struct(0, false);
+  s << "#include \"map_flow.cuh\"\n" << G.args_struct(0, false);
   s << "__device__ __forceinline__ " << T << " water_at(const Args &a, int x, int y) {\n";
   for (Node *p : P.in_rasters) {
     if (p == scan->prev[1] || !G.center_read.count(p)) continue;
@@ -2762,6 +2762,38 @@ static std::string gen_spread(Gen &G) {
       << "  if (r >= m.n) return;\n"
       << "  pj_final(((const Args *)m.args)[r], (blockIdx.x % m.slices) * blockDim.x + threadIdx.x, m.slices * blockDim.x,\n"
       << "           (int)m.round);\n"
+      << "}\n";
+  }
+  // 32-bit integer accumulations over tiles (skeleton/flow.cuh): passes A, B and C of
+  // one raster, and of many (serving windows), `per` CTAs of the launch per raster
+  if (packed) {
+    s << "struct FlowOps {\n"
+      << "  static __device__ __forceinline__ u32 water(const Args &a, int x, int y) { return (u32)water_at(a, x, y); }\n"
+      << "};\n"
+      << "struct FlowManyArgs { u64 args; s64 n; s64 per; };\n"
+      << "__device__ __forceinline__ int flow_tiles(const Args &a) {\n"
+      << "  return (a.g.W + FLOW_T - 1) / FLOW_T * ((a.g.H + FLOW_T - 1) / FLOW_T);\n"
+      << "}\n";
+    for (int fin = 0; fin < 2; fin++)
+      s << "extern \"C\" __global__ void __launch_bounds__(FLOW_NT) KNAME_flow_" << (fin ? "c" : "a")
+        << "(const __grid_constant__ Args a) {\n"
+        << "  flow_tile<FlowOps, " << (fin ? "true" : "false") << ">(a, a.in[" << kd << "], a.out[" << ko << "], (int)blockIdx.x);\n"
+        << "}\n"
+        << "extern \"C\" __global__ void __launch_bounds__(FLOW_NT) KNAME_flow_" << (fin ? "c" : "a")
+        << "_many(const __grid_constant__ FlowManyArgs m) {\n"
+        << "  const s64 r = blockIdx.x / m.per;\n"
+        << "  if (r >= m.n) return;\n"
+        << "  const Args &a = ((const Args *)m.args)[r];\n"
+        << "  const int tile = (int)(blockIdx.x - r * m.per);\n"
+        << "  if (tile < flow_tiles(a)) flow_tile<FlowOps, " << (fin ? "true" : "false") << ">(a, a.in[" << kd << "], a.out[" << ko
+        << "], tile);\n"
+        << "}\n";
+    s << "extern \"C\" __global__ void __launch_bounds__(FLOW_RIM) KNAME_flow_b(const __grid_constant__ Args a) {\n"
+      << "  flow_slots(a, (s64)blockIdx.x * FLOW_RIM + threadIdx.x);\n"
+      << "}\n"
+      << "extern \"C\" __global__ void __launch_bounds__(FLOW_RIM) KNAME_flow_b_many(const __grid_constant__ FlowManyArgs m) {\n"
+      << "  const s64 r = blockIdx.x / m.per;\n"
+      << "  if (r < m.n) flow_slots(((const Args *)m.args)[r], (blockIdx.x - r * m.per) * FLOW_RIM + threadIdx.x);\n"
       << "}\n";
   }
   const std::string kahn_fn = packed ? "spread_kahn_packed" : "spread_kahn";

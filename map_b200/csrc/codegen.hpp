@@ -120,6 +120,12 @@ constexpr int kRadialB = 32, kRadialT = 32, kRadialThreads = 64;
 size_t radial_tile_smem(int dtype);
 struct RadialScratch { size_t bytes = 0; long long tiles = 0; };
 RadialScratch radial_tile_scratch(int W, int H, int sx, int sy, long long lim, int dtype);
+// Flow accumulation over tiles (32-bit integers, skeleton/flow.cuh): whether a type
+// qualifies, the tiles of a raster and the bytes of its scratch.
+bool spread_tile_type(int dt);
+size_t spread_tiles(int W, int H);
+size_t spread_tile_scratch(int W, int H);
+constexpr int kFlowThreads = 256;
 // Pointer-jumping flow accumulation (integer types): cell limit, rounds for N
 // cells, whether a type qualifies, and the scratch bytes for N cells.
 size_t spread_pj_cells();

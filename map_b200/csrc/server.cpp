@@ -63,12 +63,14 @@ struct Req {
   std::vector<void *> scratch;
 };
 
-// Flow windows above 64 K cells with integer accumulations use pointer jumping
-// (MAP_B200_SERVE_PJ=0: the one-CTA frontier sweep instead).
-bool serve_pj() {
-  static const bool v = [] {
+// How flow windows are summed: over tiles (three launches whatever the window), or,
+// by MAP_B200_SERVE_PJ, 1: pointer jumping above 64 K cells, 0: the one-CTA frontier
+// sweep (the forms of accumulations that are no 32-bit integers).
+enum class FlowForm { TILES, JUMP, SWEEP };
+FlowForm serve_flow() {
+  static const FlowForm v = [] {
     const char *e = std::getenv("MAP_B200_SERVE_PJ");
-    return !(e && e[0] == '0');
+    return !e ? FlowForm::TILES : e[0] == '0' ? FlowForm::SWEEP : FlowForm::JUMP;
   }();
   return v;
 }
@@ -229,6 +231,8 @@ Template &Server::Impl::template_for(int type, int w, int h, bool compile) {
     } else if (g.skeleton == SK_SPREAD) {
       env.kernel(P.source, P.kname + "_prep_many", 0);
       env.kernel(P.source, P.kname + "_kahnp_many", 0);
+      if (spread_tile_type(P.core->meta.dtype))
+        for (const char *k : {"_flow_a_many", "_flow_b_many", "_flow_c_many"}) env.kernel(P.source, P.kname + k, 0);
       if (spread_pj_type(P.core->meta.dtype))
         for (const char *k : {"_pj_init_many", "_pj_step_many", "_pj_final_many"}) env.kernel(P.source, P.kname + k, 0);
       T->last_phase = std::max(T->last_phase, (int)PH_SPREAD);
@@ -273,7 +277,7 @@ void Server::Impl::run_batch(std::vector<Req *> &batch) {
     const KernelPlan *plan = nullptr;
     std::vector<unsigned char> args;
     int n = 0;
-    long long tiles = 0;   // most tiles of a radial scan
+    long long tiles = 0;   // most tiles of a radial scan or of a flow accumulation over tiles (0: other forms)
     size_t max_cells = 0;
     bool pj = false;   // flow accumulation by pointer jumping (integer type, windows above 64 K cells)
   };
@@ -377,14 +381,18 @@ void Server::Impl::run_batch(std::vector<Req *> &batch) {
           mn.tiles = std::max(mn.tiles, R.tiles);
         } else {   // SK_SPREAD
           const size_t N = (size_t)g.W * g.H;
-          const bool pj = serve_pj() && N > ((size_t)1 << 16) && spread_pj_type(P.core->meta.dtype);
+          const bool ft = serve_flow() == FlowForm::TILES && spread_tile_type(P.core->meta.dtype);
+          const bool pj = !ft && serve_flow() != FlowForm::SWEEP && N > ((size_t)1 << 16) && spread_pj_type(P.core->meta.dtype);
           // windows of one template share one launch per phase, so each form keys its own
-          Many &mn = spread[P.source + (pj ? "#pj" : "")];
+          Many &mn = spread[P.source + (ft ? "#tiles" : pj ? "#pj" : "")];
           mn.plan = &P;
           mn.pj = pj;
+          if (ft) mn.tiles = std::max(mn.tiles, (long long)spread_tiles(g.W, g.H));
           mn.max_cells = std::max(mn.max_cells, N);
           void *work = nullptr;
-          const size_t wbytes = pj ? spread_pj_scratch(N, P.core->meta.dtype) : 6 * N * sizeof(int32_t);
+          const size_t wbytes = ft   ? spread_tile_scratch(g.W, g.H)
+                                : pj ? spread_pj_scratch(N, P.core->meta.dtype)
+                                     : 6 * N * sizeof(int32_t);
           cuda_check(cudaMallocAsync(&work, wbytes, st), "cudaMallocAsync(spread work)");
           r->scratch.push_back(work);
           uint64_t aux[4] = {(uint64_t)(uintptr_t)work, (uint64_t)(uintptr_t)((int32_t *)work + 2 * N),
@@ -487,6 +495,13 @@ void Server::Impl::run_batch(std::vector<Req *> &batch) {
     cuda_check(cudaStreamWaitEvent(sp, ev[PH_LEVEL1], 0), "cudaStreamWaitEvent");
     for (auto &kv : spread) {
       Many &mn = kv.second;
+      if (mn.tiles) {
+        struct { uint64_t args; int64_t n, per; } fa{(uint64_t)(uintptr_t)dptr[bi++], mn.n, mn.tiles};
+        for (const char *pass : {"_flow_a_many", "_flow_b_many", "_flow_c_many"})
+          env.launch(env.kernel(mn.plan->source, mn.plan->kname + pass, 0), (int)(mn.n * mn.tiles), kFlowThreads, 0,
+                     (CUstream_st *)sp, &fa, sizeof fa);
+        continue;
+      }
       if (mn.pj) {
         // pointer jumping: a fixed number of rounds, `slices` CTAs per window
         const int rounds = spread_pj_rounds(mn.max_cells);

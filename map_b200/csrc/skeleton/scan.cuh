@@ -399,8 +399,9 @@ __device__ __forceinline__ int d8_index(u8 c) {
   if (c == 0 || (c & (c - 1)) != 0) return -1;
   return __ffs((int)c) - 1;
 }
-__device__ __forceinline__ int d8_dx(int d) { const int t[8] = {1, 1, 0, -1, -1, -1, 0, 1}; return t[d]; }
-__device__ __forceinline__ int d8_dy(int d) { const int t[8] = {0, 1, 1, 1, 0, -1, -1, -1}; return t[d]; }
+// x and y step of direction d, from two bits each (no table in memory)
+__device__ __forceinline__ int d8_dx(int d) { return (int)((0x901Au >> (2 * d)) & 3u) - 1; }   // 1 1 0 -1 -1 -1 0 1
+__device__ __forceinline__ int d8_dy(int d) { return (int)((0x01A9u >> (2 * d)) & 3u) - 1; }   // 0 1 1 1 0 -1 -1 -1
 
 // Downstream cell of (x, y) along its D8 code, or -1.
 __device__ __forceinline__ s64 d8_down(const RasterArg &dir, int W, int H, int x, int y) {
