@@ -1869,8 +1869,18 @@ static void gen_focal(Gen &G, std::ostringstream &body, std::ostringstream &wrap
     int align_e = 1;
     for (auto &t : P.tma) align_e = std::max(align_e, 16 / (int)dt_size(t.dtype));
     body << "  const bool inner = tile_interior<" << TW << ", " << TH << ">(a.g, t, " << hx << ", " << hy << ");\n"
-         << "  if (t.x0 % " << align_e << " == 0) {\n"
+         << "  if (t.x0 % " << align_e << " == 0 || a.aux[3] != 0) {\n"
          << "    if (gdesc) __syncthreads();   // a persistent CTA: earlier readers of the staging buffer are done\n"
+         // aux[3]: an input whose rows start on no 16-byte boundary has no tensor map
+         << "    if (a.aux[3] != 0) {\n";
+    for (int k = 0; k < nst; k++) {
+      auto &t = P.tma[k];
+      std::string ty = dt_ctype(t.dtype);
+      body << "      stage_plain<" << ty << ", " << t.box_w << ", " << t.box_h << ">((" << ty << " *)(smem + " << t.smem_off
+           << "), a.in[" << t.in_index << "], a.g, t.x0 - " << t.pad_x << ", t.y0 - " << hy << ");\n";
+    }
+    body << "      __syncthreads();\n"
+         << "    } else {\n"
          << "    if (threadIdx.x == 0) {\n"
          << "      fence_proxy_async();\n";
     for (int k = 0; k < nst; k++) body << "      if (gdesc) tensormap_acquire(&a.tm[" << k << "]);\n";
@@ -1887,6 +1897,7 @@ static void gen_focal(Gen &G, std::ostringstream &body, std::ostringstream &wrap
          << "      return false;\n"
          << "    }\n"
          << "    phase ^= 1u;\n"
+         << "    }\n"
          << "    if (!inner) {\n";
     for (int k = 0; k < nst; k++) {
       auto &t = P.tma[k];

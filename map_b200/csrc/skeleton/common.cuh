@@ -653,6 +653,16 @@ __device__ __forceinline__ bool block_exception(const Geom &g, int x, int y, int
   return (edge_y && near_bx) || (edge_x && near_by) || inner_last_x || inner_last_y;
 }
 
+// Stages a box by plain loads (zero outside the raster, as the tensor maps fill), for
+// rasters whose rows start on no 16-byte boundary. The caller synchronises.
+template <class T, int SW, int SH> __device__ __forceinline__ void stage_plain(T *s, const RasterArg &r, const Geom &g, int ox, int oy) {
+#pragma unroll 8
+  for (int i = (int)threadIdx.x; i < SW * SH; i += (int)blockDim.x) {
+    const int x = ox + i % SW, y = oy + i / SW;
+    s[i] = (unsigned)x < (unsigned)g.W && (unsigned)y < (unsigned)g.H ? ldr<T>(r, x, y) : (T)0;
+  }
+}
+
 // After a staged box of an edge tile has landed (raster cell (ox + bx, oy + by) at
 // s[by * SW + bx]), overwrites its cells outside the raster that a centre cell can
 // reach (within hx / hy of the edge) with the border rule's value: zero (dead) or
