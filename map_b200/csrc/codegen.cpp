@@ -1915,41 +1915,35 @@ static void gen_focal(Gen &G, std::ostringstream &body, std::ostringstream &wrap
     }
     if (loop_edge.empty()) loop_edge = loop.str();
     // block-mirror exceptions of staged edge tiles, recomputed by the same
-    // threads (after their own stores of the same cells) from global memory
+    // threads (after their own stores of the same cells) from the staged box
     {
       std::ostringstream fx;
       fx << "      if (block_fixup(a.g)) {\n";
+      std::string taps, call1 = "focal_cell(a";
       for (int k = 0; k < nst; k++) {
+        auto &t = P.tma[k];
         std::string ty = G.T(staged_nodes[k]);
-        fx << "        const GatherTap<" << ty << "> g" << k << "{a.in[" << G.rin.at(staged_nodes[k]) << "], &a.g};\n";
+        taps += "              const BlockTap<" + ty + ", " + std::to_string(t.box_w) + "> g" + std::to_string(k) + "((const " + ty +
+                " *)(smem + " + std::to_string(t.smem_off) + "), a.g, t.x0 - " + std::to_string(t.pad_x) + ", t.y0 - " +
+                std::to_string(hy) + ", x, y);\n";
+        call1 += ", g" + std::to_string(k);
       }
-      std::string call1 = "focal_cell(a";
-      for (int k = 0; k < nst; k++) call1 += ", g" + std::to_string(k);
-      if (quad) {
-        fx << "        const int lx = 4 * (threadIdx.x % " << qw << "), ly0 = (threadIdx.x / " << qw << ") * " << qrows << ";\n"
-           << "        for (int k = 0; k < " << qrows << "; k++)\n"
-           << "          for (int c = 0; c < 4; c++) {\n"
-           << "            const int x = t.x0 + lx + c, y = t.y0 + ly0 + k;\n"
-           << "            if (x < t.xe && y < t.ye && block_exception(a.g, x, y, " << hx << ", " << hy << "))\n"
-           << "              " << call1 << ", x, y, lx + c, ly0 + k);\n"
-           << "          }\n";
-      } else if (cpair) {
-        fx << tmap
-           << "        for (int k = 0; k < " << R << "; k++)\n"
-           << "          for (int c = 0; c < 2; c++) {\n"
-           << "            const int x = t.x0 + lx + c, y = t.y0 + ly0 + k;\n"
-           << "            if (x < t.xe && y < t.ye && block_exception(a.g, x, y, " << hx << ", " << hy << "))\n"
-           << "              " << call1 << ", x, y, lx + c, ly0 + k);\n"
-           << "          }\n";
-      } else {
-        fx << tmap
-           << "        const int x = t.x0 + lx;\n"
-           << "        for (int k = 0; k < " << rows << "; k++) {\n"
-           << "          const int y = t.y0 + ly0 + k;\n"
-           << "          if (x < t.xe && y < t.ye && block_exception(a.g, x, y, " << hx << ", " << hy << "))\n"
-           << "            " << call1 << ", x, y, lx, ly0 + k);\n"
-           << "        }\n";
-      }
+      const int cols = quad ? 4 : cpair ? 2 : 1, nr = quad ? qrows : R;
+      if (quad)
+        fx << "        const int lx = 4 * (threadIdx.x % " << qw << "), ly0 = (threadIdx.x / " << qw << ") * " << qrows << ";\n";
+      else
+        fx << tmap;
+      fx << "        for (int c = 0; c < " << cols << "; c++) {\n"
+         << "          const int x = t.x0 + lx + c;\n"
+         << "          if (x >= t.xe) break;\n"
+         << "          BlockColumn column(a.g, x, t.y0 + ly0, " << hx << ", " << hy << ");\n"
+         << "          for (int k = 0; k < " << nr << "; k++) {\n"
+         << "            const int y = t.y0 + ly0 + k;\n"
+         << "            if (column.next(y) && y < t.ye) {\n"
+         << taps << "              " << call1 << ", x, y, lx + c, ly0 + k);\n"
+         << "            }\n"
+         << "          }\n"
+         << "        }\n";
       fx << "      }\n";
       loop_edge += fx.str();
     }

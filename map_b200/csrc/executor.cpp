@@ -356,6 +356,64 @@ Executor &Executor::get() {
   return e;
 }
 
+namespace {
+
+// Tile of a standalone Local / Focal launch. Large rasters take the tiles that move
+// the most cells per second, smaller ones flatter tiles: a wide tile's threads work
+// through 16 rows one after the other while the grid leaves SMs idle or half a wave
+// over, and the edge tiles, which do more, end last. `large`: the tile of a large
+// raster whatever g's size.
+TileCfg standalone_tile(const Group &g, bool large) {
+  TileCfg cfg;
+  const FocalTune &ft = focal_tune();
+  const double cells = large ? 1e12 : (double)g.W * g.H;
+  if (g.skeleton == SK_FOCAL && focal_quad_form(g)) {
+    // packed byte form: 128 x 16 tiles of 128 threads, a warp on the 32 words of
+    // one tile row, 4 rows per thread (Life at 4096^2 with dependent launches:
+    // 1021 Gcell-updates/s, against 996 for 64 x 32 and 981 for 128 x 32 of 256)
+    cfg.tw = ft.qtw ? ft.qtw : 128;
+    cfg.th = ft.qth ? ft.qth : 16;
+    cfg.nt = ft.qnt ? ft.qnt : 128;
+  } else if (g.skeleton == SK_FOCAL) {
+    cfg.nt = 128;
+    bool flow = false;
+    for (Node *n : g.nodes) flow |= n->kind == K_FOCALFLOW;
+    if (focal_fast_shade(g)) {
+      if (cells > 262144 && cells < 6e6) {
+        // 64 x 16 tiles of 128 threads: 1500^2 9.8 us against 15.0 of the 64 x 64 ones,
+        // 2048^2 13.6 against 17.0, 3000 x 2500 under the dead border 21.5 against 21.2.
+        // Up to 512^2 the call's host side hides most of it (256^2 7.5 us either way,
+        // 512^2 7.4 against 10.1) and the large tiles stay.
+        cfg.th = 16;
+      } else {
+        // 64 x 64 tiles of 256 threads, 16 rows per thread (532 Gcells/s at 16384^2,
+        // against 530 for 32 x 128 of 256 threads and 513 for 32 x 128 of 128, the
+        // same box, with per-thread store addresses), registers capped for 6 resident
+        // CTAs per SM (533 against 521 with the 5 that 48 registers allow, the same box)
+        cfg.tw = 64;
+        cfg.th = 64;
+        cfg.nt = 256;
+        cfg.minb = 6;
+      }
+    } else if (cells < 3e6) {
+      cfg.th = 8;    // 1500^2: D8 12.1 us against 16.1 of 64 x 32, slope 11.0 against 13.7, a 3 x 3 correlation 7.9 against 11.1
+    } else if (cells < 8e6 || flow) {
+      cfg.th = 16;   // 2048^2: slope 16.3 us against 17.4, the correlation 9.8 against 11.4 (8192^2: 102 against 85); D8 8192^2 196 against 207
+    }                // else 64 x 32, 16 rows per thread
+    if (ft.nt) cfg.nt = ft.nt;
+    if (ft.tw) cfg.tw = ft.tw;
+    if (ft.th) cfg.th = ft.th;
+  } else if (g.skeleton == SK_LOCAL) {
+    if (ft.lnt) cfg.nt = ft.lnt;
+    if (ft.ltw) cfg.tw = ft.ltw;
+    if (ft.lth) cfg.th = ft.lth;
+  }
+  cfg.tile_store = g.skeleton == SK_FOCAL;   // whole-raster launches: the output tile store where it applies
+  return cfg;
+}
+
+}  // namespace
+
 Executor::Prepared Executor::prepare(const std::vector<Node *> &targets, const std::set<Node *> &tset, bool compile) {
   Prepared P;
   P.order = collect(targets);
@@ -365,41 +423,7 @@ Executor::Prepared Executor::prepare(const std::vector<Node *> &targets, const s
   std::set<std::string> seen;
   for (auto &g : P.fr.groups) {
     if (g->skeleton == SK_HOST) { P.plans[g->id].skeleton = SK_HOST; continue; }
-    // standalone focal kernels: 128 threads on a 64 x 32 tile (16 rows per thread),
-    // measured 1.5% faster than 256 threads on the hillshade and 2% on life
-    TileCfg cfg;
-    if (g->skeleton == SK_FOCAL && focal_quad_form(*g)) {
-      // packed byte form: 128 x 16 tiles of 128 threads, a warp on the 32 words of
-      // one tile row, 4 rows per thread (Life at 4096^2 with dependent launches:
-      // 1021 Gcell-updates/s, against 996 for 64 x 32 and 981 for 128 x 32 of 256)
-      const FocalTune &ft = focal_tune();
-      cfg.tw = ft.qtw ? ft.qtw : 128;
-      cfg.th = ft.qth ? ft.qth : 16;
-      cfg.nt = ft.qnt ? ft.qnt : 128;
-    } else if (g->skeleton == SK_FOCAL) {
-      cfg.nt = 128;
-      if (focal_fast_shade(*g)) {
-        // fast hillshade form: 64 x 64 tiles of 256 threads, 16 rows per thread
-        // (532 Gcells/s at 16384^2, against 530 for 32 x 128 of 256 threads and
-        // 513 for 32 x 128 of 128, the same box, with per-thread store addresses),
-        // registers capped for 6 resident CTAs per SM (533 against 521 with the
-        // 5 that 48 registers allow, the same box)
-        cfg.tw = 64;
-        cfg.th = 64;
-        cfg.nt = 256;
-        cfg.minb = 6;
-      }
-      const FocalTune &ft = focal_tune();
-      if (ft.nt) cfg.nt = ft.nt;
-      if (ft.tw) cfg.tw = ft.tw;
-      if (ft.th) cfg.th = ft.th;
-    } else if (g->skeleton == SK_LOCAL) {
-      const FocalTune &ft = focal_tune();
-      if (ft.lnt) cfg.nt = ft.lnt;
-      if (ft.ltw) cfg.tw = ft.ltw;
-      if (ft.lth) cfg.th = ft.lth;
-    }
-    cfg.tile_store = g->skeleton == SK_FOCAL;   // whole-raster launches: the output tile store where it applies
+    TileCfg cfg = standalone_tile(*g, false);
     P.plans[g->id] = generate_kernel(*g, cfg);
     if (compile && seen.insert(P.plans[g->id].source).second) {
       const std::string *src = &P.plans[g->id].source;

@@ -638,25 +638,38 @@ __device__ __forceinline__ bool focal_src(const Geom &g, int x, int y, int dx, i
 // leaves the raster past the right / bottom edge from a block that is not the
 // last one, or from a last block narrower than the halo (the reflection inside
 // it is clamped). Only cells within the halo of a raster edge qualify; staged
-// edge tiles recompute them from global memory afterwards.
+// edge tiles recompute them from the staged box afterwards.
 __device__ __forceinline__ bool block_fixup(const Geom &g) {
   return g.border == 0 && !(g.BS0 >= g.W && g.BS1 >= g.H);
 }
-__device__ __forceinline__ bool block_exception(const Geom &g, int x, int y, int hx, int hy) {
-  const int bx = x % g.BS0, by = y % g.BS1;
-  const bool near_bx = bx < hx || bx >= g.BS0 - hx || x >= g.W - hx;
-  const bool near_by = by < hy || by >= g.BS1 - hy || y >= g.H - hy;
-  const bool edge_y = y < hy || y >= g.H - hy, edge_x = x < hx || x >= g.W - hx;
-  const int lastx = (g.W - 1) / g.BS0, lasty = (g.H - 1) / g.BS1;
-  const bool inner_last_x = x >= g.W - hx && (x / g.BS0 != lastx || g.W - lastx * g.BS0 < hx);
-  const bool inner_last_y = y >= g.H - hy && (y / g.BS1 != lasty || g.H - lasty * g.BS1 < hy);
-  return (edge_y && near_bx) || (edge_x && near_by) || inner_last_x || inner_last_y;
-}
+// The test of the cells (x, y0), (x, y0 + 1), ... of a column in turn: the divisions
+// are made once per column (made per cell, they kept edge tiles running 10 us after
+// the others of a small raster had ended).
+struct BlockColumn {
+  int H, BS1, hy, by, last_y0;
+  bool edge_x, near_bx, last_x, narrow_y;
+  __device__ __forceinline__ BlockColumn(const Geom &g, int x, int y0, int hx, int hy_) : H(g.H), BS1(g.BS1), hy(hy_) {
+    const int bx = x % g.BS0, last_x0 = (g.W - 1) / g.BS0 * g.BS0;
+    by = y0 % BS1;
+    last_y0 = (H - 1) / BS1 * BS1;
+    narrow_y = H - last_y0 < hy;
+    edge_x = x < hx || x >= g.W - hx;
+    near_bx = bx < hx || bx >= g.BS0 - hx || x >= g.W - hx;
+    last_x = x >= g.W - hx && (x < last_x0 || g.W - last_x0 < hx);
+  }
+  __device__ __forceinline__ bool next(int y) {
+    const bool below = y >= H - hy, edge_y = y < hy || below;
+    const bool near_by = by < hy || by >= BS1 - hy || below;
+    const bool last_y = below && (y < last_y0 || narrow_y);
+    if (++by == BS1) by = 0;
+    return (edge_y && near_bx) || (edge_x && near_by) || last_x || last_y;
+  }
+};
 
 // Stages a box by plain loads (zero outside the raster, as the tensor maps fill), for
 // rasters whose rows start on no 16-byte boundary. The caller synchronises.
 template <class T, int SW, int SH> __device__ __forceinline__ void stage_plain(T *s, const RasterArg &r, const Geom &g, int ox, int oy) {
-#pragma unroll 8
+#pragma unroll 4
   for (int i = (int)threadIdx.x; i < SW * SH; i += (int)blockDim.x) {
     const int x = ox + i % SW, y = oy + i / SW;
     s[i] = (unsigned)x < (unsigned)g.W && (unsigned)y < (unsigned)g.H ? ldr<T>(r, x, y) : (T)0;
@@ -775,6 +788,28 @@ template <class T> __device__ __forceinline__ T __float_as_raw(float f) {
   memcpy(&r, &f, sizeof(T));
   return r;
 }
+
+// The block mirror's own reads of one cell within the halo of the raster's edge, from
+// the staged box (raster cell (ox + bx, oy + by) at s[by * SW + bx]): every source the
+// rule names lies in the raster and within the halo of the cell, so in the box. The
+// cell's block is found once for all its taps.
+template <class T, int SW> struct BlockTap {
+  const T *s;
+  int ox, oy, W, H, bx0, by0, bw, bh;
+  __device__ __forceinline__ BlockTap(const T *s_, const Geom &g, int ox_, int oy_, int x, int y)
+      : s(s_), ox(ox_), oy(oy_), W(g.W), H(g.H), bx0((x / g.BS0) * g.BS0), by0((y / g.BS1) * g.BS1) {
+    bw = min(g.BS0, W - bx0);
+    bh = min(g.BS1, H - by0);
+  }
+  __device__ __forceinline__ T tap(int x, int y, int lx, int ly, int dx, int dy) const {
+    int sx = x + dx, sy = y + dy;
+    if ((unsigned)sx >= (unsigned)W || (unsigned)sy >= (unsigned)H) {
+      sx = bx0 + reflect_idx(sx - bx0, bw);
+      sy = by0 + reflect_idx(sy - by0, bh);
+    }
+    return s[(sy - oy) * SW + (sx - ox)];
+  }
+};
 
 template <class T, int SW, int PX, int HY> struct SmemTap {
   const T *s;
