@@ -169,6 +169,31 @@ bool predict_group(const Group &g, const KernelPlan &K, std::unordered_map<Node 
   return true;
 }
 
+// Whether predict_group can hold for g whatever the scalars' values, the border and
+// the groups before: every output must come from constants and scalars alone, or
+// through an integer product with one of them.
+bool may_fold(const Group &g) {
+  if (g.skeleton != SK_LOCAL && g.skeleton != SK_FOCAL) return false;
+  std::unordered_set<Node *> members(g.nodes.begin(), g.nodes.end()), open;   // open: cells that differ
+  // a raster from outside the group may be another group's fixed output
+  for (Node *in : g.inputs)
+    if (in->meta.numdim != D0 && (in->is_input() || in->kind == K_RADIALSCAN || in->kind == K_SPREADSCAN)) open.insert(in);
+  for (Node *n : g.nodes) {
+    bool all = true, any = false;
+    for (Node *p : n->prev) {
+      if (open.count(p)) all = false;
+      else any = true;
+    }
+    const bool zero = n->kind == K_BINARY && n->op == MUL && !dt_is_float(n->meta.dtype) && any;
+    const bool cell = n->kind == K_INDEX || n->kind == K_RAND || n->kind == K_FOCALFLOW || n->kind == K_FOCALPERCENT;
+    const bool pick = n->kind == K_CONDITIONAL && !open.count(n->prev[0]) && (!open.count(n->prev[1]) || !open.count(n->prev[2]));
+    if (cell || (!all && !zero && !pick)) open.insert(n);
+  }
+  for (Node *o : g.outputs)
+    if (open.count(o)) return false;
+  return true;
+}
+
 }  // namespace
 
 std::vector<PlainJob> plain_schedule(const std::vector<std::unique_ptr<Group>> &groups, const std::vector<KernelPlan> &plans) {
@@ -473,37 +498,55 @@ void Executor::find_chains(Prepared &P, const std::set<Node *> &tset) {
   }
 }
 
-std::shared_ptr<Executor::Prepared> Executor::prepare_cached(const std::vector<Node *> &targets,
-                                                             const std::set<Node *> &tset) {
+std::shared_ptr<Executor::Prepared> Executor::prepare_cached(const std::vector<Node *> &targets) {
   Runtime &rt = Runtime::get();
-  std::string key = std::to_string(rt.exec_mode) + "," + std::to_string(rt.paired_cells) + "," +
-                    std::to_string(rt.algebraic_rewrite) + ";";   // prediction runs per evaluation (not cached)
-  for (Node *t : targets) key += std::to_string(t->id) + ",";
-  key += ";";
-  for (Node *t : tset) key += std::to_string(t->id) + ",";
-  auto sig = [](const Prepared &P) {
-    std::vector<char> v;
-    for (Node *n : P.order)
-      if (n->meta.numdim == D0) v.push_back(n->has_value ? 1 : 0);
-    return v;
+  // prediction runs per evaluation (not cached)
+  std::vector<int> key = {rt.exec_mode, (int)rt.paired_cells, (int)rt.algebraic_rewrite};
+  key.reserve(3 + targets.size());
+  for (Node *t : targets) key.push_back(t->id);
+  uint64_t h = 1469598103934665603ull;
+  for (int k : key) h = (h ^ (uint32_t)k) * 1099511628211ull;
+  auto same_sig = [](const CacheEntry &c) {
+    for (size_t i = 0; i < c.d0sig.size(); i++)
+      if ((c.P->d0[i]->has_value ? 1 : 0) != c.d0sig[i]) return false;
+    return true;
   };
-  auto it = cache_.find(key);
-  if (it != cache_.end() && it->second.epoch == rt.epoch && it->second.d0sig == sig(*it->second.P)) {
-    it->second.used = ++cache_tick_;
-    return it->second.P;
+  auto known = cache_.equal_range(h);
+  for (auto it = known.first; it != known.second;) {
+    CacheEntry &c = it->second;
+    if (c.key == key) {
+      if (c.epoch == rt.epoch && same_sig(c)) {
+        c.used = ++cache_tick_;
+        return c.P;
+      }
+      it = cache_.erase(it);
+    } else {
+      ++it;
+    }
   }
+  const std::set<Node *> tset(targets.begin(), targets.end());
   auto P = std::make_shared<Prepared>(prepare(targets, tset, true));
+  for (auto &g : P->fr.groups) {
+    if (g->skeleton != SK_HOST) P->need_device = true;
+    if (may_fold(*g)) P->foldable = true;
+  }
+  for (Node *t : targets)
+    if (t->meta.numdim != D0) P->need_device = true;
+  for (Node *n : P->order)
+    if (n->meta.numdim == D0) P->d0.push_back(n);
   if (cache_.size() >= 64) {   // evict the least recently used entry
     auto lru = cache_.begin();
     for (auto c = cache_.begin(); c != cache_.end(); ++c)
       if (c->second.used < lru->second.used) lru = c;
     cache_.erase(lru);
   }
-  CacheEntry &e = cache_[key];
+  CacheEntry e;
   e.P = P;
-  e.d0sig = sig(*P);
+  e.key = std::move(key);
+  for (Node *n : P->d0) e.d0sig.push_back(n->has_value ? 1 : 0);
   e.epoch = rt.epoch;
   e.used = ++cache_tick_;
+  cache_.emplace(h, std::move(e));
   return P;
 }
 
@@ -654,17 +697,13 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
   for (auto &s : sinks) targets.push_back(s.node);
   for (Node *t : targets)
     if (!rt.owns(t)) throw MapError("evaluate: unknown node");
-  std::set<Node *> tset(targets.begin(), targets.end());
-  std::shared_ptr<Prepared> PP = prepare_cached(targets, tset);
+  std::shared_ptr<Prepared> PP = prepare_cached(targets);
   const Prepared &P = *PP;
   last = EvalStats();
   last.groups = (int)P.fr.groups.size();
   const int launches0 = env.launches();
 
-  bool need_device = false;
-  for (auto &g : P.fr.groups) if (g->skeleton != SK_HOST) need_device = true;
-  for (Node *t : targets) if (t->meta.numdim != D0) need_device = true;
-  if (!need_device) {
+  if (!P.need_device) {
     for (auto &g : P.fr.groups) {
       Node *n = g->nodes[0];
       n->value = host_eval(n);
@@ -905,7 +944,7 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
   // groups whose every output is one known value (Predictor): filled, not launched
   std::unordered_map<Node *, Variant> fixed;
   std::vector<char> predicted(P.fr.groups.size(), 0), filled(P.fr.groups.size(), 0);
-  if (rt.prediction)
+  if (rt.prediction && P.foldable)
     for (auto &gp : P.fr.groups)
       predicted[gp->id] = predict_group(*gp, P.plans[gp->id], fixed, rt.border) ? 1 : 0;
   // a chain runs when none of its groups is predicted
@@ -1170,8 +1209,7 @@ void Executor::evaluate_rows(const std::vector<Node *> &targets_in, const std::v
     if (!rt.owns(t)) throw MapError("evalRows: unknown node");
     if (t->meta.numdim != D2) throw MapError("evalRows: every output is a 2-D raster");
   }
-  std::set<Node *> tset(targets.begin(), targets.end());
-  std::shared_ptr<Prepared> PP = prepare_cached(targets, tset);
+  std::shared_ptr<Prepared> PP = prepare_cached(targets);
   const Prepared &P = *PP;
   for (Node *n : P.order)
     if (n->kind == K_WRITE) throw MapError("evalRows: a program with file writes runs whole");

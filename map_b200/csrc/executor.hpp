@@ -126,6 +126,9 @@ class Executor {
     };
     std::vector<Chain> chains;
     std::vector<int> chain_of;   // per group: its chain, or -1
+    bool foldable = false;       // some group's outputs may all be fixed (predict_group is worth a look)
+    bool need_device = false;    // some group runs on the device
+    std::vector<Node *> d0;      // the scalar nodes of `order`
   };
   Prepared prepare(const std::vector<Node *> &targets, const std::set<Node *> &tset, bool compile);
   static void find_chains(Prepared &P, const std::set<Node *> &tset);
@@ -133,13 +136,14 @@ class Executor {
   // scalar values, no node destroyed since) reuse their fusion and kernel plans.
   struct CacheEntry {
     std::shared_ptr<Prepared> P;
+    std::vector<int> key;      // launch mode, packed and rewritten forms, target ids
     std::vector<char> d0sig;   // has_value of every D0 node of P.order
     uint64_t epoch = 0;
     uint64_t used = 0;
   };
-  std::map<std::string, CacheEntry> cache_;
+  std::unordered_multimap<uint64_t, CacheEntry> cache_;   // by a hash of the key
   uint64_t cache_tick_ = 0;
-  std::shared_ptr<Prepared> prepare_cached(const std::vector<Node *> &targets, const std::set<Node *> &tset);
+  std::shared_ptr<Prepared> prepare_cached(const std::vector<Node *> &targets);
   // Row-band streaming of host-to-host Local / Focal programs; false (and no
   // work done) when the program does not qualify.
   bool evaluate_streamed(const Prepared &P, const std::vector<Node *> &targets, const std::vector<Sink> &sinks);
