@@ -404,11 +404,11 @@ TileCfg standalone_tile(const Group &g, bool large) {
     bool flow = false;
     for (Node *n : g.nodes) flow |= n->kind == K_FOCALFLOW;
     if (focal_fast_shade(g)) {
-      if (cells > 262144 && cells < 6e6) {
-        // 64 x 16 tiles of 128 threads: 1500^2 9.8 us against 15.0 of the 64 x 64 ones,
-        // 2048^2 13.6 against 17.0, 3000 x 2500 under the dead border 21.5 against 21.2.
-        // Up to 512^2 the call's host side hides most of it (256^2 7.5 us either way,
-        // 512^2 7.4 against 10.1) and the large tiles stay.
+      if ((g.H < 512 || cells > 262144) && cells < 6e6) {
+        // 64 x 16 tiles of 128 threads: 256^2 7.5 us a call against 10.3 of the 64 x 64
+        // ones (fewer than eight rows of tall tiles leave most SMs idle), 1500^2 9.8
+        // against 15.0, 2048^2 13.6 against 17.0, 3000 x 2500 under the dead border
+        // 21.5 against 21.2
         cfg.th = 16;
       } else {
         // 64 x 64 tiles of 256 threads, 16 rows per thread (532 Gcells/s at 16384^2,
@@ -947,11 +947,13 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
   if (rt.prediction && P.foldable)
     for (auto &gp : P.fr.groups)
       predicted[gp->id] = predict_group(*gp, P.plans[gp->id], fixed, rt.border) ? 1 : 0;
-  // a chain runs when none of its groups is predicted
+  // a chain runs when none of its groups is predicted and its tiles fit a grid
   std::vector<char> chained(P.chains.size(), 1);
-  for (size_t c = 0; c < P.chains.size(); c++)
+  for (size_t c = 0; c < P.chains.size(); c++) {
+    if (P.fr.groups[P.chains[c].groups[0]]->H > kMaxGridY * (kRuleRowsSmall - 2 * kRuleMaxGensSmall)) chained[c] = 0;
     for (int id : P.chains[c].groups)
       if (predicted[id]) chained[c] = 0;
+  }
   auto run_chain = [&](const Prepared::Chain &c) {
     const Group &g = *P.fr.groups[c.groups.front()];
     const KernelPlan &first = P.plans[g.id], &last_plan = P.plans[c.groups.back()];
