@@ -303,7 +303,7 @@ std::vector<unsigned char> pack_args(const Group &g, const KernelPlan &K, const 
   bool plain = false;
   for (const TmaSpec &t : K.tma) {
     const DevRaster &r = get(K.in_rasters[t.in_index]);
-    plain |= r.rows == 0 && (((uintptr_t)r.ptr & 15) != 0 || (r.pitch & 15) != 0);
+    plain |= K.tile_store && r.rows == 0 && (((uintptr_t)r.ptr & 15) != 0 || (r.pitch & 15) != 0);
   }
   for (size_t k = 0; !plain && k < K.tma.size(); k++) {
     const TmaSpec &t = K.tma[k];

@@ -642,7 +642,18 @@ __device__ __forceinline__ bool focal_src(const Geom &g, int x, int y, int dx, i
 __device__ __forceinline__ bool block_fixup(const Geom &g) {
   return g.border == 0 && !(g.BS0 >= g.W && g.BS1 >= g.H);
 }
-// The test of the cells (x, y0), (x, y0 + 1), ... of a column in turn: the divisions
+__device__ __forceinline__ bool block_exception(const Geom &g, int x, int y, int hx, int hy) {
+  const int bx = x % g.BS0, by = y % g.BS1;
+  const bool near_bx = bx < hx || bx >= g.BS0 - hx || x >= g.W - hx;
+  const bool near_by = by < hy || by >= g.BS1 - hy || y >= g.H - hy;
+  const bool edge_y = y < hy || y >= g.H - hy, edge_x = x < hx || x >= g.W - hx;
+  const int lastx = (g.W - 1) / g.BS0, lasty = (g.H - 1) / g.BS1;
+  const bool inner_last_x = x >= g.W - hx && (x / g.BS0 != lastx || g.W - lastx * g.BS0 < hx);
+  const bool inner_last_y = y >= g.H - hy && (y / g.BS1 != lasty || g.H - lasty * g.BS1 < hy);
+  return (edge_y && near_bx) || (edge_x && near_by) || inner_last_x || inner_last_y;
+}
+
+// The same test of the cells (x, y0), (x, y0 + 1), ... of a column in turn: the divisions
 // are made once per column (made per cell, they kept edge tiles running 10 us after
 // the others of a small raster had ended).
 struct BlockColumn {
