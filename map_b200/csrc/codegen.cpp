@@ -2052,8 +2052,9 @@ static std::string gen_zonal(Gen &G) {
   // raster outputs: a thread loads V = 16 / es cells of a row at a time, all of its
   // tile's vectors first, and folds them into `sets` accumulators of each reduction
   // in turn (shorter chains of dependent additions, and of roundings). Other tiles
-  // take one cell at a time. stats.py's seven reductions of an 8192^2 raster: 4-byte
-  // loads and one accumulator left the loads waiting on each other.
+  // take one cell at a time. stats.py at 8192^2 (two passes, squares and cubes by
+  // products): 734 -> 268 us; its first pass, seven reductions with a division per
+  // cell, takes 109 us, 72% of the issue slots, its second 70 us.
   int es = 0;
   bool vec = G.outk.empty() && !P.in_rasters.empty();
   for (Node *p : P.in_rasters) {
