@@ -823,14 +823,35 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
     }
     return false;
   };
+  // Whether output o may be written over the device inputs that its sink's memory
+  // meets: every group that reads such an input has run before o's group starts, or
+  // is o's group itself and element-wise on the very same cells. All other groups
+  // read cells (halos, other fronts, the water a second time) that some CTA of the
+  // same launch may already have written. (A chain keeps its own first read and last
+  // write apart, and its groups before the last run before.)
+  auto in_place = [&](Node *o, const Sink &s) {
+    auto holds = [](const std::vector<Node *> &v, Node *n) { return std::find(v.begin(), v.end(), n) != v.end(); };
+    for (Node *n : P.order) {
+      if (n->kind != K_DEVIN || !meets(n->dev->ptr, n->dev->pitch, n->meta.H(), s.dev, s.dev_pitch, s.node->meta.H())) continue;
+      const bool same_cells = n->dev->ptr == s.dev && n->dev->pitch == s.dev_pitch && dt_size(n->meta.dtype) == dt_size(o->meta.dtype);
+      bool after = false;   // o's group, or a later one
+      for (auto &gp : P.fr.groups) {
+        const KernelPlan &K = P.plans[gp->id];
+        const bool own = holds(K.out_rasters, o);
+        after |= own || rt.exec_mode != EXEC_FUSED;
+        if (after && holds(K.in_rasters, n) && !(own && gp->skeleton == SK_LOCAL && same_cells)) return false;
+      }
+    }
+    return true;
+  };
   std::function<DevRaster(Node *)> alloc_out = [&](Node *o) -> DevRaster {
     auto ds = dev_sink.find(o);
     if (ds != dev_sink.end()) {
       const Sink *s = ds->second;
-      // straight into the caller's buffer; rows on no 16-byte boundary only where no
-      // other group reads the raster back
+      // straight into the caller's buffer, where that may be written in place; rows on
+      // no 16-byte boundary only where no other group reads the raster back
       const long long es = (long long)dt_size(o->meta.dtype);
-      const bool aligned = ((uintptr_t)s->dev & 127) == 0 && (s->dev_pitch & 15) == 0;
+      const bool aligned = ((uintptr_t)s->dev & 127) == 0 && (s->dev_pitch & 15) == 0 && in_place(o, *s);
       const bool apart = (uintptr_t)s->dev % (uintptr_t)es == 0 && s->dev_pitch % es == 0 && readers(o) == 0 && !in_chain(o) &&
                          !meets_input(*s);
       if ((aligned || apart) && s->dev_pitch >= (long long)o->meta.W() * es) {
