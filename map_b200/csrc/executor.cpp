@@ -376,6 +376,32 @@ std::vector<unsigned char> pack_args(const Group &g, const KernelPlan &K, const 
 // Local / Focal tiles are launched in pieces of this many tile rows.
 constexpr int kMaxGridY = 65535;
 
+// Whether ph rows of pp bytes from p on share memory with qh rows of qp bytes from q on.
+static bool meets(const void *p, long long pp, long long ph, const void *q, long long qp, long long qh) {
+  const uintptr_t a = (uintptr_t)p, b = (uintptr_t)q;
+  return a < b + (uintptr_t)(qp * qh) && b < a + (uintptr_t)(pp * ph);
+}
+
+// Whether output o may be written over device input n, whose memory its own meets:
+// every group that reads n has run before o's group starts (`ordered`: groups run one
+// after the other), or is o's group itself and element-wise on the very same cells.
+// All other groups read cells (halos, other fronts, the water a second time) that
+// some CTA of the same launch may already have written. (A chain keeps its own first
+// read and last write apart, and its groups before the last run before.)
+static bool writable_over(const FusionResult &fr, const std::vector<KernelPlan> &plans, Node *o, Node *n, bool same_cells,
+                          bool ordered) {
+  auto holds = [](const std::vector<Node *> &v, Node *m) { return std::find(v.begin(), v.end(), m) != v.end(); };
+  same_cells &= dt_size(n->meta.dtype) == dt_size(o->meta.dtype);
+  bool after = !ordered;   // o's group, or a later one
+  for (auto &gp : fr.groups) {
+    const KernelPlan &K = plans[gp->id];
+    const bool own = holds(K.out_rasters, o);
+    after |= own;
+    if (after && holds(K.in_rasters, n) && !(own && gp->skeleton == SK_LOCAL && same_cells)) return false;
+  }
+  return true;
+}
+
 Executor &Executor::get() {
   static Executor e;
   return e;
@@ -748,10 +774,6 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
   };
   // whether a device input's memory meets a sink's: such rasters are read and written
   // apart from each other (a copy of the input, or of the output)
-  auto meets = [](const void *p, long long pp, int ph, const void *q, long long qp, int qh) {
-    const uintptr_t a = (uintptr_t)p, b = (uintptr_t)q;
-    return a < b + (uintptr_t)(qp * qh) && b < a + (uintptr_t)(pp * ph);
-  };
   auto meets_sink = [&](const DevRaster &r) {
     for (const Sink &s : sinks)
       if (s.dev && meets(r.ptr, r.pitch, r.H, s.dev, s.dev_pitch, s.node->meta.H())) return true;
@@ -823,25 +845,11 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
     }
     return false;
   };
-  // Whether output o may be written over the device inputs that its sink's memory
-  // meets: every group that reads such an input has run before o's group starts, or
-  // is o's group itself and element-wise on the very same cells. All other groups
-  // read cells (halos, other fronts, the water a second time) that some CTA of the
-  // same launch may already have written. (A chain keeps its own first read and last
-  // write apart, and its groups before the last run before.)
   auto in_place = [&](Node *o, const Sink &s) {
-    auto holds = [](const std::vector<Node *> &v, Node *n) { return std::find(v.begin(), v.end(), n) != v.end(); };
-    for (Node *n : P.order) {
-      if (n->kind != K_DEVIN || !meets(n->dev->ptr, n->dev->pitch, n->meta.H(), s.dev, s.dev_pitch, s.node->meta.H())) continue;
-      const bool same_cells = n->dev->ptr == s.dev && n->dev->pitch == s.dev_pitch && dt_size(n->meta.dtype) == dt_size(o->meta.dtype);
-      bool after = false;   // o's group, or a later one
-      for (auto &gp : P.fr.groups) {
-        const KernelPlan &K = P.plans[gp->id];
-        const bool own = holds(K.out_rasters, o);
-        after |= own || rt.exec_mode != EXEC_FUSED;
-        if (after && holds(K.in_rasters, n) && !(own && gp->skeleton == SK_LOCAL && same_cells)) return false;
-      }
-    }
+    for (Node *n : P.order)
+      if (n->kind == K_DEVIN && meets(n->dev->ptr, n->dev->pitch, n->meta.H(), s.dev, s.dev_pitch, s.node->meta.H()) &&
+          !writable_over(P.fr, P.plans, o, n, n->dev->ptr == s.dev && n->dev->pitch == s.dev_pitch, rt.exec_mode == EXEC_FUSED))
+        return false;
     return true;
   };
   std::function<DevRaster(Node *)> alloc_out = [&](Node *o) -> DevRaster {
@@ -1281,6 +1289,16 @@ void Executor::evaluate_rows(const std::vector<Node *> &targets_in, const std::v
   }
   std::map<Node *, const Sink *> sink_of;
   for (const Sink &s : sinks) sink_of[s.node] = &s;
+  // a sink in the memory of an input is written at the end unless its group may write there
+  auto in_place = [&](const Sink &s) {
+    for (Node *n : R.inputs) {
+      const DevData &d = *n->dev;
+      if (!meets(d.ptr, d.pitch, d.rows ? d.rows : H, s.dev, s.dev_pitch, y1 - y0)) continue;
+      const bool same_cells = (char *)d.ptr + (long long)(y0 - d.row0) * d.pitch == (char *)s.dev && d.pitch == s.dev_pitch;
+      if (!writable_over(P.fr, P.plans, s.node, n, same_cells, true)) return false;
+    }
+    return true;
+  };
   std::vector<void *> allocs;
   std::vector<std::pair<const Sink *, Node *>> copies;
   try {
@@ -1292,7 +1310,7 @@ void Executor::evaluate_rows(const std::vector<Node *> &targets_in, const std::v
       r.H = H;
       auto sk = sink_of.find(n);
       if (sk != sink_of.end() && R.need[R.producer[n]] == 0 && ((uintptr_t)sk->second->dev & 15) == 0 &&
-          (sk->second->dev_pitch & 15) == 0) {
+          (sk->second->dev_pitch & 15) == 0 && in_place(*sk->second)) {
         // written straight into the caller's rows [y0, y1)
         r.pitch = sk->second->dev_pitch;
         r.org = y0;

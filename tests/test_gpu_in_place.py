@@ -87,3 +87,27 @@ def test_radial_into_its_raster(fresh, shape, obs):
     pitch = (4 * shape[1] + 127) // 128 * 128
     _check(M, dem, M.F32, lambda x: W.viewshed(x, list(obs), 5.0), pitch, 0, 0)
     _check(M, dem, M.F32, lambda x: M.rmin(x, list(obs)), pitch, 0, 128)
+
+
+@pytest.mark.parametrize("border", [0, 2])
+@pytest.mark.parametrize("band,shift", [(False, 0), (True, 0), (False, 2), (True, -1)])
+def test_rows_into_the_input(fresh, border, band, shift):
+    # rows [40, 90) evaluated into the rows `shift` further on of the raster, or of the
+    # band of rows around them, that they are computed from
+    import torch
+    M = fresh
+    M.set_border(border)
+    h, w, y0, y1 = 150, 333, 40, 90
+    dem = synth.fbm_dem(h, w, seed=14)
+    pitch = (4 * w + 127) // 128 * 128
+    for program in (W.hillshade, lambda x: x * 3.0 + 1.0, lambda x: M.convolve(M.convolve(x, W3), W3) + x):
+        want = M.to_numpy(program(M.from_numpy(dem, bs=[64, 48])))[y0:y1]
+        ra, rb = (y0 - 4, y1 + 4) if band else (0, h)
+        raw = torch.zeros((rb - ra, pitch // 4), dtype=torch.float32, device="cuda")
+        raw[:, :w].copy_(torch.from_numpy(dem[ra:rb]).cuda())
+        torch.cuda.synchronize()
+        x = (M.from_device_rows(raw.data_ptr(), pitch, [w, h], M.F32, ra, rb - ra, bs=[64, 48]) if band
+             else M.from_device(raw.data_ptr(), pitch, [w, h], M.F32, [64, 48]))
+        at = y0 - ra + shift
+        M.eval_rows([program(x)], [(raw.data_ptr() + at * pitch, pitch)], y0, y1)
+        assert np.array_equal(raw[at:at + y1 - y0, :w].cpu().numpy(), want)
