@@ -1422,6 +1422,13 @@ bool Executor::evaluate_streamed(const Prepared &P, const std::vector<Node *> &t
     B = std::max(32, B / 32 * 32);
     if ((long long)H < 4LL * B) return false;
   }
+  // a result in the memory of an input: a band's download may overwrite rows that the
+  // next band still uploads, unless every band reads just the rows that it writes
+  for (const Sink &s : sinks)
+    for (Node *n : host_in) {
+      const long long to = (long long)W * (long long)dt_size(s.node->meta.dtype), from = (long long)W * (long long)dt_size(n->meta.dtype);
+      if (meets(s.host, to, H, n->host->ptr, from, H) && !(M == 0 && s.host == n->host->ptr && to == from)) return false;
+    }
 
   CudaEnv &env = CudaEnv::get();
   cudaStream_t st = (cudaStream_t)env.stream();

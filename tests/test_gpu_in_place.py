@@ -111,3 +111,25 @@ def test_rows_into_the_input(fresh, border, band, shift):
         at = y0 - ra + shift
         M.eval_rows([program(x)], [(raw.data_ptr() + at * pitch, pitch)], y0, y1)
         assert np.array_equal(raw[at:at + y1 - y0, :w].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("rows", [40, 257])
+@pytest.mark.parametrize("shift", [0, 3])
+def test_host_raster_into_its_own_memory(fresh, rows, shift):
+    # streamed bands: a focal program into its input's rows runs whole, an element-wise
+    # one on the very same rows in bands
+    M = fresh
+    h, w = 777, 523
+    dem = synth.fbm_dem(h, w, seed=15)
+    for program, bands in ((W.hillshade, 0), (lambda x: x * 2.0 + 1.0, 0 if shift else -(-h // rows))):
+        M.set_stream_rows(-1)
+        want = M.to_numpy(program(M.from_numpy(dem, bs=[128, 128])))
+        mem = np.zeros((h + shift, w), np.float32)
+        mem[:h] = dem
+        M.set_stream_rows(rows)
+        try:
+            M.to_numpy(program(M.from_numpy(mem[:h], bs=[128, 128], copy=False)), out=mem[shift:])
+            assert M.last_band_count() == bands
+        finally:
+            M.set_stream_rows(0)
+        assert np.array_equal(mem[shift:], want)
