@@ -40,6 +40,7 @@
 #include "codegen.hpp"
 #include "cuda_env.hpp"
 #include "executor.hpp"
+#include "stream_memory.hpp"
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -164,16 +165,15 @@ void run_scan_group(const Group &g, const KernelPlan &P, std::unordered_map<Node
     uint64_t aux[4] = {(uint64_t)scan->coord.arr[0], (uint64_t)scan->coord.arr[1], (uint64_t)lim, 0};
     if (tiled) {
       const RadialScratch R = radial_tile_scratch(g.W, g.H, scan->coord.arr[0], scan->coord.arr[1], lim, scan->meta.dtype);
-      void *work = nullptr;
-      cuda_check(cudaMallocAsync(&work, R.bytes, st), "cudaMallocAsync(radial work)");
-      cuda_check(cudaMemsetAsync(work, 0, R.bytes, st), "memset");
+      StreamMemory work(st);
+      cuda_check(work.alloc(R.bytes), "allocation of the radial scan's scratch");
+      cuda_check(cudaMemsetAsync(work.ptr(), 0, R.bytes, st), "memset");
       KernelHandle kt = env.kernel(P.source, P.kname + "_tiles", P.smem_bytes);
       const long long cap = (long long)env.sm_count() * std::max(1, env.occupancy(kt, kRadialThreads, P.smem_bytes));
-      aux[3] = (uint64_t)(uintptr_t)work;
+      aux[3] = (uint64_t)(uintptr_t)work.ptr();
       auto at = pack_args(g, P, get, bufs, 0, 0, g.W, g.H, aux);
       env.launch(kt, (int)std::max<long long>(1, std::min(cap, R.tiles)), kRadialThreads, P.smem_bytes, (CUstream_st *)st, at.data(),
                  at.size());
-      cuda_check(cudaFreeAsync(work, st), "cudaFreeAsync");
       return;
     }
     auto a = pack_args(g, P, get, bufs, 0, 0, g.W, g.H, aux);
@@ -195,11 +195,11 @@ void run_scan_group(const Group &g, const KernelPlan &P, std::unordered_map<Node
   const size_t N = (size_t)g.W * g.H;
   if (N >= (size_t)1 << 31) throw MapError("spreadScan: raster too large");
   if (N > kSpreadKahnCells && N <= spread_pj_cells() && spread_pj_type(scan->meta.dtype)) {
-    void *work = nullptr;
-    cuda_check(cudaMallocAsync(&work, spread_pj_scratch(N, scan->meta.dtype), st), "cudaMallocAsync(spread work)");
+    StreamMemory work(st);
+    cuda_check(work.alloc(spread_pj_scratch(N, scan->meta.dtype)), "allocation of the flow accumulation's scratch");
     const int rounds = spread_pj_rounds(N);
     const int grid = (int)std::max<size_t>(1, std::min<size_t>((2 * N + 255) / 256, (size_t)env.sm_count() * 8));
-    uint64_t aux[4] = {(uint64_t)(uintptr_t)work, 0, 0, 0};
+    uint64_t aux[4] = {(uint64_t)(uintptr_t)work.ptr(), 0, 0, 0};
     auto a = pack_args(g, P, get, bufs, 0, 0, g.W, g.H, aux);
     env.launch(env.kernel(P.source, P.kname + "_pj_init", 0), grid, 256, 0, (CUstream_st *)st, a.data(), a.size());
     KernelHandle ks = env.kernel(P.source, P.kname + "_pj_step", 0);
@@ -211,27 +211,25 @@ void run_scan_group(const Group &g, const KernelPlan &P, std::unordered_map<Node
     aux[1] = (uint64_t)rounds;
     auto af = pack_args(g, P, get, bufs, 0, 0, g.W, g.H, aux);
     env.launch(env.kernel(P.source, P.kname + "_pj_final", 0), grid, 256, 0, (CUstream_st *)st, af.data(), af.size());
-    cuda_check(cudaFreeAsync(work, st), "cudaFreeAsync");
     return;
   }
   // Over tiles at every size: 64^2 33 us against 42 of the one-CTA sweep, 256^2 38
   // against 365, 700 x 500 50 against 98 of the walks, 2048^2 103 against 500-544,
   // 8000^2 1.1 ms against 7.4 (directions included).
   if (spread_tile_type(scan->meta.dtype) && Runtime::get().exec_mode == EXEC_FUSED) {
-    void *work = nullptr;
-    cuda_check(cudaMallocAsync(&work, spread_tile_scratch(g.W, g.H), st), "cudaMallocAsync(spread work)");
-    uint64_t aux[4] = {(uint64_t)(uintptr_t)work, 0, 0, 0};
+    StreamMemory work(st);
+    cuda_check(work.alloc(spread_tile_scratch(g.W, g.H)), "allocation of the flow accumulation's scratch");
+    uint64_t aux[4] = {(uint64_t)(uintptr_t)work.ptr(), 0, 0, 0};
     auto a = pack_args(g, P, get, bufs, 0, 0, g.W, g.H, aux);
     for (const char *pass : {"_flow_a", "_flow_b", "_flow_c"})
       env.launch(env.kernel(P.source, P.kname + pass, 0), (int)spread_tiles(g.W, g.H), kFlowThreads, 0, (CUstream_st *)st, a.data(),
                  a.size());
-    cuda_check(cudaFreeAsync(work, st), "cudaFreeAsync");
     return;
   }
-  void *work = nullptr;
-  cuda_check(cudaMallocAsync(&work, 6 * N * sizeof(int32_t), st), "cudaMallocAsync(spread work)");
-  uint64_t aux[4] = {(uint64_t)(uintptr_t)work, (uint64_t)(uintptr_t)((int32_t *)work + 2 * N),
-                     (uint64_t)(uintptr_t)((int32_t *)work + 4 * N), (uint64_t)(N + 1)};
+  StreamMemory work(st);
+  cuda_check(work.alloc(6 * N * sizeof(int32_t)), "allocation of the flow accumulation's scratch");
+  int32_t *const w = (int32_t *)work.ptr();
+  uint64_t aux[4] = {(uint64_t)(uintptr_t)w, (uint64_t)(uintptr_t)(w + 2 * N), (uint64_t)(uintptr_t)(w + 4 * N), (uint64_t)(N + 1)};
   auto a = pack_args(g, P, get, bufs, 0, 0, g.W, g.H, aux);
   if (N <= kSpreadKahnCells) {
     // one CTA, frontier by frontier: the lowest latency up to 64 K cells
@@ -242,7 +240,6 @@ void run_scan_group(const Group &g, const KernelPlan &P, std::unordered_map<Node
     env.launch(ki, grid, 256, 0, (CUstream_st *)st, a.data(), a.size());
     env.launch(kh, grid, 256, 0, (CUstream_st *)st, a.data(), a.size());
   }
-  cuda_check(cudaFreeAsync(work, st), "cudaFreeAsync");
 }
 
 }  // namespace mapb

@@ -2,6 +2,7 @@
 #include "executor.hpp"
 #include "binfile.hpp"
 #include "cuda_env.hpp"
+#include "stream_memory.hpp"
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -1004,11 +1005,20 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
     KernelHandle kh = env.kernel(c.plan.source, c.plan.kname + (small ? "_gens_s" : "_gens"), c.plan.smem_bytes);
     std::unordered_map<Node *, DevRaster> io;
     std::function<DevRaster &(Node *)> bound = [&](Node *n) -> DevRaster & { return io.at(n); };
+    StreamMemory held0(st), held1(st), *const held[2] = {&held0, &held1};
     DevRaster tmp[2], cur = src;
     for (int i = 0; launches > 0; i++, launches--) {
       const int k = (left + launches - 1) / launches;
       left -= k;
-      if (launches > 1 && !tmp[i & 1].ptr) tmp[i & 1] = alloc_raster(U8, g.W, g.H);
+      if (launches > 1 && !tmp[i & 1].ptr) {
+        DevRaster &r = tmp[i & 1];
+        r.dtype = U8;
+        r.W = g.W;
+        r.H = g.H;
+        r.pitch = pitch_for(g.W, U8);
+        cuda_check(held[i & 1]->alloc((size_t)r.pitch * g.H), "allocation of a rule chain's generation");
+        r.ptr = held[i & 1]->ptr();
+      }
       io[c.plan.in_rasters[0]] = cur;
       io[c.plan.out_rasters[0]] = cur = launches > 1 ? tmp[i & 1] : dst;
       const uint64_t aux[4] = {(uint64_t)k, 0, 0, 0};
@@ -1019,8 +1029,6 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
       else
         env.launch_2d(kh, tx, ty, kRuleThreads, c.plan.smem_bytes, (CUstream_st *)st, a.data());
     }
-    for (const DevRaster &r : tmp)
-      if (r.ptr) cuda_check(cudaFreeAsync(r.ptr, st), "cudaFreeAsync");
   };
   auto fill_predicted = [&](const Group &g, const KernelPlan &K) {
     ensure_outputs(g, K);
