@@ -121,10 +121,13 @@ size_t radial_tile_smem(int dtype);
 struct RadialScratch { size_t bytes = 0; long long tiles = 0; };
 RadialScratch radial_tile_scratch(int W, int H, int sx, int sy, long long lim, int dtype);
 // Flow accumulation over tiles (32-bit integers, skeleton/flow.cuh): whether a type
-// qualifies, the tiles of a raster and the bytes of its scratch.
+// qualifies, the tiles of a raster, the bytes of its scratch, and whether the rim slots
+// (256 a tile) of a raster can be numbered in 31 bits. Rasters of one to three columns
+// or rows reach that limit below 2^31 cells.
 bool spread_tile_type(int dt);
-size_t spread_tiles(int W, int H);
-size_t spread_tile_scratch(int W, int H);
+constexpr size_t spread_tiles(int W, int H) { return ((size_t)W + 63) / 64 * (((size_t)H + 63) / 64); }
+constexpr size_t spread_tile_scratch(int W, int H) { return spread_tiles(W, H) * 256 * 16; }
+constexpr bool spread_tiles_fit(int W, int H) { return spread_tiles(W, H) * 256 < ((size_t)1 << 31); }
 constexpr int kFlowThreads = 256;
 // Pointer-jumping flow accumulation (integer types): cell limit, rounds for N
 // cells, whether a type qualifies, and the scratch bytes for N cells.

@@ -82,8 +82,6 @@ int spread_pj_rounds(size_t N) {
 bool spread_pj_type(int dt) { return dt == S32 || dt == U32 || dt == S64 || dt == U64; }
 size_t spread_pj_scratch(size_t N, int dt) { return 4 * N * (sizeof(int32_t) + dt_size(dt)); }
 bool spread_tile_type(int dt) { return dt == S32 || dt == U32; }
-size_t spread_tiles(int W, int H) { return (size_t)((W + 63) / 64) * (size_t)((H + 63) / 64); }
-size_t spread_tile_scratch(int W, int H) { return spread_tiles(W, H) * 256 * 16; }
 // radial scans of rasters at least this wide or tall use CTA clusters per octant
 constexpr int kRadialClusterDim = 2048;
 constexpr int kRadialCluster = 8;
@@ -215,8 +213,9 @@ void run_scan_group(const Group &g, const KernelPlan &P, std::unordered_map<Node
   }
   // Over tiles at every size: 64^2 33 us against 42 of the one-CTA sweep, 256^2 38
   // against 365, 700 x 500 50 against 98 of the walks, 2048^2 103 against 500-544,
-  // 8000^2 1.1 ms against 7.4 (directions included).
-  if (spread_tile_type(scan->meta.dtype) && Runtime::get().exec_mode == EXEC_FUSED) {
+  // 8000^2 1.1 ms against 7.4 (directions included). Rasters too thin for the slots'
+  // numbers walk.
+  if (spread_tile_type(scan->meta.dtype) && spread_tiles_fit(g.W, g.H) && Runtime::get().exec_mode == EXEC_FUSED) {
     StreamMemory work(st);
     cuda_check(work.alloc(spread_tile_scratch(g.W, g.H)), "allocation of the flow accumulation's scratch");
     uint64_t aux[4] = {(uint64_t)(uintptr_t)work.ptr(), 0, 0, 0};

@@ -381,7 +381,7 @@ void Server::Impl::run_batch(std::vector<Req *> &batch) {
           mn.tiles = std::max(mn.tiles, R.tiles);
         } else {   // SK_SPREAD
           const size_t N = (size_t)g.W * g.H;
-          const bool ft = serve_flow() == FlowForm::TILES && spread_tile_type(P.core->meta.dtype);
+          const bool ft = serve_flow() == FlowForm::TILES && spread_tile_type(P.core->meta.dtype) && spread_tiles_fit(g.W, g.H);
           const bool pj = !ft && serve_flow() != FlowForm::SWEEP && N > ((size_t)1 << 16) && spread_pj_type(P.core->meta.dtype);
           // windows of one template share one launch per phase, so each form keys its own
           Many &mn = spread[P.source + (ft ? "#tiles" : pj ? "#pj" : "")];
