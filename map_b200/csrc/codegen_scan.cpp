@@ -11,8 +11,8 @@
 // front at a time with a cluster barrier between fronts; 8 B per cell would take 21
 // us of HBM: the 2250 fronts' chain (about 65 ns each with the exchange between
 // strips) and the issue of two IEEE divisions and square roots per cell bound it.
-// A tile reads cells that its neighbours write, so a raster evaluated into the
-// memory of one of its inputs is swept front by front instead: one CTA per octant,
+// A scan whose scratch (an eighth of the raster's bytes, up to four times them for
+// rasters one cell wide) cannot be had is swept front by front, which needs none: one CTA per octant,
 // a front's cells spread over the CTA's threads, the previous and current fronts in
 // shared memory when both fit (radial_front_smem, up to 200 KiB); for rasters at
 // least kRadialClusterDim cells across, the octant runs on a cluster of
@@ -91,20 +91,16 @@ size_t radial_front_smem(int W, int H, int dtype) {
   return b <= (size_t)200 * 1024 ? b : 0;                          // larger: fronts re-read from the output
 }
 
-// Whether an output of the group shares memory with one of its inputs (a caller
-// may evaluate a raster into its own buffer).
-static bool overlap(const Group &g, const KernelPlan &P, std::unordered_map<Node *, DevRaster> &bufs,
-                    const std::function<DevRaster &(Node *)> &get) {
-  for (Node *o : P.out_rasters) {
-    const DevRaster &d = bufs.at(o);
-    const uintptr_t d0 = (uintptr_t)d.ptr, d1 = d0 + (uintptr_t)(d.pitch * g.H);
-    for (Node *in : P.in_rasters) {
-      const DevRaster &r = get(in);
-      const uintptr_t r0 = (uintptr_t)r.ptr, r1 = r0 + (uintptr_t)(r.pitch * g.H);
-      if (d0 < r1 && r0 < d1) return true;
-    }
-  }
-  return false;
+// The most scratch that the tiles of one scan may take: MAP_B200_SCAN_SCRATCH bytes,
+// read at each scan, or whatever the pool has. A scan whose tiles cannot have theirs
+// runs in the form that needs none (radial: front by front) or, thin, less (flow: walks).
+static bool tile_scratch(StreamMemory &work, size_t bytes) {
+  const char *e = std::getenv("MAP_B200_SCAN_SCRATCH");
+  if (e && bytes > std::strtoull(e, nullptr, 10)) return false;
+  const cudaError_t r = work.alloc(bytes);
+  if (r == cudaErrorMemoryAllocation) return false;
+  cuda_check(r, "allocation of a scan's scratch");
+  return true;
 }
 
 size_t radial_tile_smem(int dtype) {
@@ -137,9 +133,18 @@ void run_scan_group(const Group &g, const KernelPlan &P, std::unordered_map<Node
   CudaEnv &env = CudaEnv::get();
   cudaStream_t st = (cudaStream_t)env.stream();
   Node *scan = P.core;
+  StreamMemory work(st);
+  RadialScratch R;
+  long long lim = -1;
+  bool tiled = false;
+  if (scan->kind == K_RADIALSCAN) {
+    if (scan->radius > 0) lim = (long long)scan->radius;
+    R = radial_tile_scratch(g.W, g.H, scan->coord.arr[0], scan->coord.arr[1], lim, scan->meta.dtype);
+    tiled = tile_scratch(work, R.bytes);
+  }
   for (Node *o : P.out_rasters) {
     if (bufs.count(o)) continue;
-    if (o == scan && g.scan_private && scan->kind == K_RADIALSCAN) {
+    if (o == scan && g.scan_private && tiled) {
       DevRaster none;   // the tiled form keeps no raster that only the group itself reads
       none.dtype = o->meta.dtype;
       none.W = g.W;
@@ -150,21 +155,13 @@ void run_scan_group(const Group &g, const KernelPlan &P, std::unordered_map<Node
     }
   }
   if (scan->kind == K_RADIALSCAN) {
-    const bool tiled = !overlap(g, P, bufs, get);
-    if (!tiled && !bufs.at(scan).ptr) bufs[scan] = alloc_out(scan);
-    long long lim = -1;
-    if (scan->radius > 0) {
-      lim = (long long)scan->radius;
+    if (lim >= 0)
       for (Node *o : P.out_rasters) {
         DevRaster &r = bufs.at(o);
         if (r.ptr) cuda_check(cudaMemset2DAsync(r.ptr, r.pitch, 0xFF, (size_t)r.W * dt_size(r.dtype), r.H, st), "memset");
       }
-    }
     uint64_t aux[4] = {(uint64_t)scan->coord.arr[0], (uint64_t)scan->coord.arr[1], (uint64_t)lim, 0};
     if (tiled) {
-      const RadialScratch R = radial_tile_scratch(g.W, g.H, scan->coord.arr[0], scan->coord.arr[1], lim, scan->meta.dtype);
-      StreamMemory work(st);
-      cuda_check(work.alloc(R.bytes), "allocation of the radial scan's scratch");
       cuda_check(cudaMemsetAsync(work.ptr(), 0, R.bytes, st), "memset");
       KernelHandle kt = env.kernel(P.source, P.kname + "_tiles", P.smem_bytes);
       const long long cap = (long long)env.sm_count() * std::max(1, env.occupancy(kt, kRadialThreads, P.smem_bytes));
@@ -193,7 +190,6 @@ void run_scan_group(const Group &g, const KernelPlan &P, std::unordered_map<Node
   const size_t N = (size_t)g.W * g.H;
   if (N >= (size_t)1 << 31) throw MapError("spreadScan: raster too large");
   if (N > kSpreadKahnCells && N <= spread_pj_cells() && spread_pj_type(scan->meta.dtype)) {
-    StreamMemory work(st);
     cuda_check(work.alloc(spread_pj_scratch(N, scan->meta.dtype)), "allocation of the flow accumulation's scratch");
     const int rounds = spread_pj_rounds(N);
     const int grid = (int)std::max<size_t>(1, std::min<size_t>((2 * N + 255) / 256, (size_t)env.sm_count() * 8));
@@ -215,9 +211,8 @@ void run_scan_group(const Group &g, const KernelPlan &P, std::unordered_map<Node
   // against 365, 700 x 500 50 against 98 of the walks, 2048^2 103 against 500-544,
   // 8000^2 1.1 ms against 7.4 (directions included). Rasters too thin for the slots'
   // numbers walk.
-  if (spread_tile_type(scan->meta.dtype) && spread_tiles_fit(g.W, g.H) && Runtime::get().exec_mode == EXEC_FUSED) {
-    StreamMemory work(st);
-    cuda_check(work.alloc(spread_tile_scratch(g.W, g.H)), "allocation of the flow accumulation's scratch");
+  if (spread_tile_type(scan->meta.dtype) && spread_tiles_fit(g.W, g.H) && Runtime::get().exec_mode == EXEC_FUSED &&
+      tile_scratch(work, spread_tile_scratch(g.W, g.H))) {
     uint64_t aux[4] = {(uint64_t)(uintptr_t)work.ptr(), 0, 0, 0};
     auto a = pack_args(g, P, get, bufs, 0, 0, g.W, g.H, aux);
     for (const char *pass : {"_flow_a", "_flow_b", "_flow_c"})
@@ -225,7 +220,6 @@ void run_scan_group(const Group &g, const KernelPlan &P, std::unordered_map<Node
                  a.size());
     return;
   }
-  StreamMemory work(st);
   cuda_check(work.alloc(6 * N * sizeof(int32_t)), "allocation of the flow accumulation's scratch");
   int32_t *const w = (int32_t *)work.ptr();
   uint64_t aux[4] = {(uint64_t)(uintptr_t)w, (uint64_t)(uintptr_t)(w + 2 * N), (uint64_t)(uintptr_t)(w + 4 * N), (uint64_t)(N + 1)};
