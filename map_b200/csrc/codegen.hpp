@@ -126,7 +126,7 @@ RadialScratch radial_tile_scratch(int W, int H, int sx, int sy, long long lim, i
 // or rows reach that limit below 2^31 cells.
 bool spread_tile_type(int dt);
 constexpr size_t spread_tiles(int W, int H) { return ((size_t)W + 63) / 64 * (((size_t)H + 63) / 64); }
-constexpr size_t spread_tile_scratch(int W, int H) { return spread_tiles(W, H) * 256 * 16; }
+constexpr size_t spread_tile_scratch(int W, int H) { return spread_tiles(W, H) * (256 * 16 + 512); }
 constexpr bool spread_tiles_fit(int W, int H) { return spread_tiles(W, H) * 256 < ((size_t)1 << 31); }
 constexpr int kFlowThreads = 256;
 // Pointer-jumping flow accumulation (integer types): cell limit, rounds for N

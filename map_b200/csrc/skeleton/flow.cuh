@@ -9,15 +9,18 @@
 //   C. every tile adds the water that enters at its rim to the sums of pass A (kept
 //      in the output) down the paths it takes, and takes each cell's own water off.
 // Integer sums are exact in any order, modulo the type's width, so the result is the
-// whole-raster walks' bit for bit; cells on a cycle of codes, and rim cells that take
-// water from one, never complete and hold zero, as there.
+// whole-raster walks' bit for bit. Cells on a cycle of codes never complete and hold
+// zero, as there; a cell has one code, so no path leaves a cycle and all other cells
+// complete. Cycles inside a tile are found by pass A's pointers and marked in the
+// scratch, those that cross tiles by the slots that pass B leaves pending.
 //
 // 2048^2 (fBm, 4.2 M cells): 42 + 7 + 38 us for the passes, against 46 + 540 us for
 // counting and walking the whole raster, whose longest path of one L2 atomic per cell
 // bounds it. The tiles' passes are bound by shared-memory latency at four CTAs per SM
 // (62 registers; five or six measured the same). Tried for the tiles: walks with
 // counts 200 us a pass (a thread's longest walk sets the tile's time), doubling in
-// pass C too 56 us.
+// pass C too 56 us. Random codes, full of cycles, at 2048^2: 124 us, against 279 of the
+// whole-raster walks and 642 when tiles with a cycle took walks with counts.
 #pragma once
 #include "map_scan.cuh"
 
@@ -29,12 +32,14 @@
 #define FLOW_CYCLE (-2)                // the enter slot that marks a tile with a cycle of codes
 #define FLOW_EXIT 0x4000               // the end is a rim cell whose water leaves the tile
 
-// Scratch at aux[0] (host: flow_scratch): per rim slot the water that leaves there
-// and its pending pushes (u64), the slot it enters by in the next tile (s32), and
-// for a slot where water enters the one where it leaves again (s32, -1: it stays).
+// Scratch at aux[0] (host: spread_tile_scratch): per rim slot the water that leaves
+// there and its pending pushes (u64), the slot it enters by in the next tile (s32), and
+// for a slot where water enters the one where it leaves again (s32, -1: it stays); per
+// tile with a cycle of codes a bit per cell, set for the cycles' cells.
 struct FlowScratch {
   u64 *pk;
   s32 *enter, *leave;
+  u32 *loop;
   int tx, ty;
 };
 template <class ARGS> __device__ __forceinline__ FlowScratch flow_scratch(const ARGS &a) {
@@ -45,6 +50,7 @@ template <class ARGS> __device__ __forceinline__ FlowScratch flow_scratch(const 
   f.pk = (u64 *)a.aux[0];
   f.enter = (s32 *)(f.pk + n);
   f.leave = f.enter + n;
+  f.loop = (u32 *)(f.leave + n);
   return f;
 }
 // Rim slot of cell (lx, ly) of a w x h tile: top row, bottom row, left and right column.
@@ -58,12 +64,13 @@ __device__ __forceinline__ int flow_slot(const FlowScratch &f, int W, int H, int
          flow_rim(x - cx * FLOW_T, y - cy * FLOW_T, min(FLOW_T, W - cx * FLOW_T), min(FLOW_T, H - cy * FLOW_T));
 }
 
-// Sums a tile whose paths all end (no cycle of codes): doubling. In round r every
-// cell adds what it holds to the cell 2^r steps down its path, if the path is that
-// long, and takes over that cell's pointer; afterwards sum[c] is the water of c and
-// of all cells above it, and next[c] names the end of its path. Cells of a thread
-// are independent, so a round's shared-memory latencies overlap. False when a
-// path has not ended after enough rounds for the longest (a cycle).
+// Sums a tile by doubling: in round r every cell adds what it holds to the cell 2^r
+// steps down its path, if the path is that long, and takes over that cell's pointer;
+// afterwards sum[c] is the water of c and of all cells above it (c on no cycle of
+// codes), and next[c] names the end of its path. Cells of a thread are independent, so
+// a round's shared-memory latencies overlap. False when a path has not ended after
+// rounds for twice the longest: its pointer is then a cell of the cycle that it runs
+// into, and the cycle's own cells' pointers are all of its cells.
 template <int PER> __device__ __forceinline__ bool flow_double(u32 *sum, u16 *next, int tid) {
   u32 s[PER];
   u16 n[PER];
@@ -93,40 +100,11 @@ template <int PER> __device__ __forceinline__ bool flow_double(u32 *sum, u16 *ne
   return false;
 }
 
-// Sums a tile of any codes: counts of pending pushes (bytes), and walks from the
-// cells nothing flows into. Cells on a cycle keep a count and hold no sum.
-template <int PER> __device__ __forceinline__ void flow_walks(u32 *sum, const u16 *next, u32 *cnt, int tid) {
-  u32 sources = 0u;   // bit k: cell tid + k * FLOW_NT
-  for (int k = 0; k < PER; ++k)
-    if (((const u8 *)cnt)[tid + k * FLOW_NT] == 0u) sources |= 1u << k;
-  __syncthreads();
-  int c = -1;
-  for (;;) {
-    if (c < 0) {
-      if (!sources) break;
-      c = tid + (__ffs((int)sources) - 1) * FLOW_NT;
-      sources &= sources - 1;
-    }
-    const int to = next[c];
-    if (to & FLOW_DONE) {
-      c = -1;
-      continue;
-    }
-    const u32 v = *(volatile u32 *)&sum[c];
-    atomicAdd(&sum[to], v);
-    __threadfence_block();   // the push is seen before its count
-    const u32 old = atomicSub(&cnt[to >> 2], 1u << (8 * (to & 3)));
-    c = ((old >> (8 * (to & 3))) & 255u) == 1u ? to : -1;
-    __threadfence_block();
-  }
-  __syncthreads();
-}
-
 template <class OPS, bool FINAL, class ARGS>
 __device__ __forceinline__ void flow_tile(const ARGS &a, const RasterArg &D, const RasterArg &O, int tile) {
   constexpr int CW = FLOW_T + 32, PAD = 16, CELLS = FLOW_T * FLOW_T, PER = CELLS / FLOW_NT;
   __shared__ __align__(16) u8 code[CW * (FLOW_T + 2)];   // rows y0 - 1 .. y0 + 64, columns x0 - 16 .. x0 + 79
-  __shared__ u32 sum[CELLS], cnt[CELLS / 4];
+  __shared__ u32 sum[CELLS], loop[CELLS / 32];   // loop: bits of the cells on cycles
   __shared__ u16 next[CELLS];
   __shared__ u32 pending[FLOW_RIM];
   const FlowScratch f = flow_scratch(a);
@@ -185,65 +163,34 @@ __device__ __forceinline__ void flow_tile(const ARGS &a, const RasterArg &D, con
     rim = ly > 0 && ly < h - 1 && (side == 2 || w > 1);
   }
   const int slot = tile * FLOW_RIM + tid, cell = ly * FLOW_T + lx;
-  // the neighbours (bit j) whose code leads to cell (cx, cy), inside the tile or outside
-  auto feeders = [&](int cx, int cy, bool inside) {
-    const u8 *const p = code + (cy + 1) * CW + cx + PAD;
-    u32 m = 0u;
+  // the neighbours (bit j) outside the tile whose code leads to the rim cell
+  u32 enter = 0u;
+  if (rim) {
+    const u8 *const p = code + (ly + 1) * CW + lx + PAD;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const int nx = cx - d8_dx(j), ny = cy - d8_dy(j);
+      const int nx = lx - d8_dx(j), ny = ly - d8_dy(j);
       const bool in = (unsigned)nx < (unsigned)w && (unsigned)ny < (unsigned)h;
-      if (p[-d8_dx(j) - CW * d8_dy(j)] == (u8)(1 << j) && in == inside) m |= 1u << j;
+      if (p[-d8_dx(j) - CW * d8_dy(j)] == (u8)(1 << j) && !in) enter |= 1u << j;
     }
-    return m;
-  };
-  const u32 enter = rim ? feeders(lx, ly, false) : 0u;
-  u32 blocked = 0u, inflow = 0u;
-  if (FINAL)
-    for (u32 m = enter; m; m &= m - 1) {
-      const int j = __ffs((int)m) - 1;
-      const u64 v = f.pk[flow_slot(f, W, H, x0 + lx - d8_dx(j), y0 + ly - d8_dy(j))];
-      if ((u32)v == 0u || (u32)v == FLOW_SOURCE) inflow += (u32)(v >> 32);
-      else ++blocked;
-    }
-  // codes with a cycle are counted; otherwise pass A doubles, and pass C adds what
-  // enters at a rim cell to the sums of that cell and of those down its path
-  bool counted = FINAL ? __syncthreads_or(blocked != 0u || f.enter[tile * FLOW_RIM + FLOW_RIM - 1] == FLOW_CYCLE) : false;
-  __syncthreads();
+  }
+  auto mark = [&](int c) { atomicOr(&loop[c >> 5], 1u << (c & 31)); };
+  auto marked = [&](int c) { return (*(volatile u32 *)&loop[c >> 5] >> (c & 31) & 1u) != 0u; };
+  if (tid < CELLS / 32) loop[tid] = 0u;
   if (!FINAL) {
-    counted = !flow_double<PER>(sum, next, tid);
-  } else if (!counted) {
-    if (inflow)
-      for (int c = cell;; c = next[c]) {
-        atomicAdd(&sum[c], inflow);
-        if (next[c] & FLOW_DONE) break;
+    __syncthreads();
+    const bool cyclic = !flow_double<PER>(sum, next, tid);
+    if (cyclic) {
+      for (int k = 0; k < PER; ++k) {
+        const u16 n = next[tid + k * FLOW_NT];
+        if (!(n & FLOW_DONE)) mark(n);
       }
-    __syncthreads();
-  }
-  if (counted) {
-    __syncthreads();
-    for (int k = 0; k < PER; ++k) {
-      const int c = tid + k * FLOW_NT, cx = c % FLOW_T, cy = c / FLOW_T;
-      const bool in = cx < w && cy < h;
-      sum[c] = in ? OPS::water(a, x0 + cx, y0 + cy) : 0u;
-      next[c] = step(c, cx, cy);
-      ((u8 *)cnt)[c] = in ? (u8)__popc(feeders(cx, cy, true)) : (u8)255;
+      __syncthreads();
+      if (tid < CELLS / 32) f.loop[(s64)tile * (CELLS / 32) + tid] = loop[tid];
     }
-    __syncthreads();
-    if (rim) {
-      sum[cell] += inflow;
-      ((u8 *)cnt)[cell] += (u8)blocked;
-    }
-    __syncthreads();
-    flow_walks<PER>(sum, next, cnt, tid);
-  }
-  if (!FINAL) {
-    __syncthreads();
     // where water that enters at a rim cell leaves the tile
     if (enter) {
-      int e = cell, n = 0;
-      while (!(next[e] & FLOW_DONE) && ++n <= CELLS) e = next[e];
-      const u16 end = next[e];
+      const u16 end = next[cell];
       if ((end & FLOW_DONE) && (end & FLOW_EXIT)) {
         const int at = end & (CELLS - 1), r = flow_rim(at % FLOW_T, at / FLOW_T, w, h);
         atomicAdd(&pending[r], (u32)__popc(enter));
@@ -260,18 +207,53 @@ __device__ __forceinline__ void flow_tile(const ARGS &a, const RasterArg &D, con
       f.pk[slot] = (u64)sum[cell] << 32 | (pending[tid] ? pending[tid] : FLOW_SOURCE);
     }
     // (the last slot is no cell's: the tile's cycle mark)
-    f.enter[slot] = counted && tid == FLOW_RIM - 1 ? FLOW_CYCLE : into;
+    f.enter[slot] = cyclic && tid == FLOW_RIM - 1 ? FLOW_CYCLE : into;
 #pragma unroll 4
     for (int k = 0; k < PER; ++k) {
       const int i = tid + k * FLOW_NT, cx = i % FLOW_T, cy = i / FLOW_T;
       if (cx < w && cy < h) *cell_ptr<u32>(O, x0 + cx, y0 + cy) = sum[i];
     }
   } else {
+    // the water that enters at the rim cell; slots still pending lie on a cycle, and
+    // so do the cells down the path from where they enter
+    u32 inflow = 0u;
+    bool blocked = false;
+    for (u32 m = enter; m; m &= m - 1) {
+      const int j = __ffs((int)m) - 1;
+      const u64 v = f.pk[flow_slot(f, W, H, x0 + lx - d8_dx(j), y0 + ly - d8_dy(j))];
+      if ((u32)v == 0u || (u32)v == FLOW_SOURCE) inflow += (u32)(v >> 32);
+      else blocked = true;
+    }
+    const bool cyclic = f.enter[tile * FLOW_RIM + FLOW_RIM - 1] == FLOW_CYCLE;
+    const bool cycles = __syncthreads_or(blocked || cyclic);
+    if (cyclic) {
+      if (tid < CELLS / 32) loop[tid] = f.loop[(s64)tile * (CELLS / 32) + tid];
+      __syncthreads();
+    }
+    if (!cycles) {
+      if (inflow)
+        for (int c = cell;; c = next[c]) {
+          atomicAdd(&sum[c], inflow);
+          if (next[c] & FLOW_DONE) break;
+        }
+    } else if (inflow || blocked) {
+      // (apart: with the marks in them the usual walks took up to a third longer)
+      int c = cell;
+      for (int n = 0; n < CELLS; ++n) {
+        if (cyclic && marked(c)) break;
+        atomicAdd(&sum[c], inflow);
+        if (blocked) mark(c);
+        const u16 to = next[c];
+        if (to & FLOW_DONE) break;
+        c = to;
+      }
+    }
+    __syncthreads();
 #pragma unroll 4
     for (int k = 0; k < PER; ++k) {
       const int i = tid + k * FLOW_NT, cx = i % FLOW_T, cy = i / FLOW_T;
       if (cx >= w || cy >= h) continue;
-      const bool whole = !counted || ((const u8 *)cnt)[i] == 0u;
+      const bool whole = !cycles || !marked(i);
       *cell_ptr<u32>(O, x0 + cx, y0 + cy) = whole ? sum[i] - OPS::water(a, x0 + cx, y0 + cy) : 0u;
     }
   }
