@@ -834,7 +834,10 @@ int ma_zoneStatsNoAlloc(const void *value, long long value_pitch, const void *zo
 
 int ma_nodeCount(void) { return (int)Runtime::get().nodes.size(); }
 void ma_collectGarbage(void) {
-  void_call([&] { Runtime::get().collect_garbage(); });
+  void_call([&] {
+    Runtime::get().collect_garbage();
+    Executor::get().release_scratch();
+  });
 }
 
 }  // extern "C"

@@ -2970,7 +2970,7 @@ bool generate_rule(const Group &g, const std::string &kname, KernelPlan &P) {
       k = it->second;
     }
   }
-  if (!k.rule) return false;
+  if (!k.rule || !G.quadable()) return false;
   const uint32_t born = k.born, survive = k.survive;
   std::ostringstream s;
   s << "#include \"map_rule.cuh\"\n" << G.args_struct(0, false)
@@ -2987,7 +2987,10 @@ bool generate_rule(const Group &g, const std::string &kname, KernelPlan &P) {
   s << "    return r;\n  }\n"
     << "  template <class F0> static __device__ __forceinline__ u8 cell(const Args &a, const F0 &f0, int x, int y) {\n"
     << "    const int lx = 0, ly = 0;\n"
-    << G.center_loads(false) << G.body(false) << "    return (u8)(" << G.val(P.out_rasters[0]) << ");\n  }\n};\n";
+    << G.center_loads(false) << G.body(false) << "    return (u8)(" << G.val(P.out_rasters[0]) << ");\n  }\n"
+    << "  template <class F0> static __device__ __forceinline__ u32 cell4(const Args &a, const F0 &f0, int ly) {\n"
+    << "    const int lx = 0;\n"
+    << G.center_loads4() << G.body4() << "    return q4_pack_u8(" << G.val4(P.out_rasters[0]) << ");\n  }\n};\n";
   for (int small = 0; small < 2; small++)
     s << "extern \"C\" __global__ void __launch_bounds__(" << kRuleThreads << ") KNAME_gens" << (small ? "_s" : "")
       << "(const __grid_constant__ Args a) {\n"
@@ -3000,7 +3003,7 @@ bool generate_rule(const Group &g, const std::string &kname, KernelPlan &P) {
   while ((pos = src.find("KNAME")) != std::string::npos) src.replace(pos, 5, P.kname);
   P.source = src;
   P.threads = kRuleThreads;
-  P.smem_bytes = 2 * 288 * 160;   // RULE_SMEM
+  P.smem_bytes = 2 * kRuleRows * 32 * 4;   // a tile's rows of words, two generations
   return true;
 }
 

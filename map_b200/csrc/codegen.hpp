@@ -82,6 +82,10 @@ bool generate_rule(const Group &g, const std::string &kname, KernelPlan &P);   /
 // Columns, rows and generations of a tile of the rule kernels (KNAME_gens: 192
 // rows, KNAME_gens_s: 64, of which a row per generation is lost at both ends).
 constexpr int kRuleCols = 992, kRuleRows = 192, kRuleRowsSmall = 64, kRuleThreads = 512, kRuleMaxGens = 16, kRuleMaxGensSmall = 12;
+// Scratch of the rule kernels: lock words (RULE_SLOTS) and `slots` areas for tiles of
+// `rows` rows whose cells are other bytes than zero and one (RULE_BYTES).
+constexpr int kRuleSlots = 2048;
+constexpr size_t rule_scratch(int rows, int slots) { return 4 * (size_t)kRuleSlots + (size_t)slots * 2 * rows * 1056; }
 
 // Tuning overrides of the standalone Local / Focal skeletons, read once from the
 // environment variable MAP_B200_FOCAL_TUNE ("key=value,..."; the keys are the

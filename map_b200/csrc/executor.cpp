@@ -715,6 +715,28 @@ void Executor::sync() {
   }
 }
 
+void *Executor::rule_memory(size_t bytes) {
+  if (rule_cap_ < bytes) {
+    cudaStream_t st = (cudaStream_t)CudaEnv::get().stream();
+    release_scratch();
+    StreamMemory fresh(st);
+    const cudaError_t e = fresh.alloc(bytes);
+    if (e == cudaErrorMemoryAllocation) return nullptr;
+    cuda_check(e, "allocation of a rule chain's scratch");
+    cuda_check(cudaMemsetAsync(fresh.ptr(), 0, 4 * (size_t)kRuleSlots, st), "memset");
+    rule_kept_ = fresh.release();
+    rule_cap_ = bytes;
+  }
+  return rule_kept_;
+}
+
+void Executor::release_scratch() {
+  std::lock_guard<std::recursive_mutex> lk(Runtime::get().mtx);
+  if (rule_kept_) cudaFreeAsync(rule_kept_, (cudaStream_t)CudaEnv::get().stream());
+  rule_kept_ = nullptr;
+  rule_cap_ = 0;
+}
+
 void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector<Sink> &sinks, bool async) {
   const double t0 = now_ms();
   Runtime &rt = Runtime::get();
@@ -984,7 +1006,8 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
     for (int id : P.chains[c].groups)
       if (predicted[id]) chained[c] = 0;
   }
-  auto run_chain = [&](const Prepared::Chain &c) {
+  // false (nothing done): no scratch memory for the tiles
+  auto run_chain = [&](const Prepared::Chain &c) -> bool {
     const Group &g = *P.fr.groups[c.groups.front()];
     const KernelPlan &first = P.plans[g.id], &last_plan = P.plans[c.groups.back()];
     Node *in = first.in_rasters[0], *out = last_plan.out_rasters[0];
@@ -993,10 +1016,13 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
     const DevRaster dst = bufs.at(out);
     int left = (int)c.groups.size();
     // 16 generations of a 192-row tile cost it a sixth of its rows; rasters that give
-    // fewer such tiles than half the SMs take tiles of 64 rows and 12 generations.
+    // fewer such tiles than half the SMs take tiles of 64 rows and 12 generations, and so
+    // do short chains, which lose few rows: 2 generations of zeros and ones at 4096^2 10.1
+    // us against 10.8, of other bytes 37.5 against 55.7 (a launch each: 31.5); 4
+    // generations 13.0 against 13.9 and 40.4 against 59.5 (a launch each: 65.7).
     const int tx = (g.W + kRuleCols - 1) / kRuleCols;
     auto tiles = [&](int rows, int k) { return (long long)tx * ((g.H + rows - 2 * k - 1) / (rows - 2 * k)); };
-    const bool small = tiles(kRuleRows, kRuleMaxGens) * 2 < env.sm_count();
+    const bool small = left <= 4 || tiles(kRuleRows, kRuleMaxGens) * 2 < env.sm_count();
     const int rows = small ? kRuleRowsSmall : kRuleRows, most = small ? kRuleMaxGensSmall : kRuleMaxGens;
     // a launch reads its neighbours' input cells: none writes what it reads
     const uintptr_t s0 = (uintptr_t)src.ptr, d0 = (uintptr_t)dst.ptr;
@@ -1007,6 +1033,9 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
     std::function<DevRaster &(Node *)> bound = [&](Node *n) -> DevRaster & { return io.at(n); };
     StreamMemory held0(st), held1(st), *const held[2] = {&held0, &held1};
     DevRaster tmp[2], cur = src;
+    const int slots = (int)std::min<long long>(std::min(2 * env.sm_count(), kRuleSlots), tiles(rows, (left + launches - 1) / launches));
+    void *const cells = rule_memory(rule_scratch(rows, slots));
+    if (!cells) return false;
     for (int i = 0; launches > 0; i++, launches--) {
       const int k = (left + launches - 1) / launches;
       left -= k;
@@ -1021,7 +1050,7 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
       }
       io[c.plan.in_rasters[0]] = cur;
       io[c.plan.out_rasters[0]] = cur = launches > 1 ? tmp[i & 1] : dst;
-      const uint64_t aux[4] = {(uint64_t)k, 0, 0, 0};
+      const uint64_t aux[4] = {(uint64_t)k, (uint64_t)(uintptr_t)cells, (uint64_t)slots, 0};
       auto a = pack_args(g, c.plan, bound, io, 0, 0, g.W, g.H, aux);
       const int ty = (g.H + rows - 2 * k - 1) / (rows - 2 * k);
       if (rt.dependent_launch)
@@ -1029,6 +1058,7 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
       else
         env.launch_2d(kh, tx, ty, kRuleThreads, c.plan.smem_bytes, (CUstream_st *)st, a.data());
     }
+    return true;
   };
   auto fill_predicted = [&](const Group &g, const KernelPlan &K) {
     ensure_outputs(g, K);
@@ -1051,7 +1081,11 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
         if (predicted[g.id]) { fill_predicted(g, K); continue; }
         if (P.chain_of[g.id] >= 0 && chained[P.chain_of[g.id]]) {
           const Prepared::Chain &c = P.chains[P.chain_of[g.id]];
-          if (c.groups.back() == g.id) run_chain(c);
+          if (c.groups.back() == g.id && !run_chain(c))
+            for (int id : c.groups) {   // a launch per generation
+              ensure_outputs(*P.fr.groups[id], P.plans[id]);
+              launch_region(*P.fr.groups[id], P.plans[id], 0, 0, g.W, g.H);
+            }
           continue;
         }
         if (g.skeleton == SK_RADIAL || g.skeleton == SK_SPREAD) {

@@ -112,6 +112,8 @@ class Executor {
   std::vector<PlainJob> schedule_for(const std::vector<Node *> &targets);
   EvalStats last;
   void sync();
+  // Gives back the scratch kept between evaluations.
+  void release_scratch();
 
  private:
   struct Prepared {
@@ -144,6 +146,13 @@ class Executor {
   std::unordered_multimap<uint64_t, CacheEntry> cache_;   // by a hash of the key
   uint64_t cache_tick_ = 0;
   std::shared_ptr<Prepared> prepare_cached(const std::vector<Node *> &targets);
+  // Scratch of the rule chains' tiles (rule_scratch), zero lock words first. Kept between
+  // evaluations, all on the engine's stream under the runtime's lock: an allocation and
+  // its release cost a small chain 2.5 us of its 15. Bounded by two tiles per SM, 120 MB;
+  // released with the unused nodes (release_scratch). Null: no memory.
+  void *rule_memory(size_t bytes);
+  void *rule_kept_ = nullptr;
+  size_t rule_cap_ = 0;
   // Row-band streaming of host-to-host Local / Focal programs; false (and no
   // work done) when the program does not qualify.
   bool evaluate_streamed(const Prepared &P, const std::vector<Node *> &targets, const std::vector<Sink> &sinks);

@@ -27,6 +27,12 @@ class StreamMemory {
     return e;
   }
   void *ptr() const { return p_; }
+  // the memory, no longer given back by this object
+  void *release() {
+    void *p = p_;
+    p_ = nullptr;
+    return p;
+  }
 
  private:
   cudaStream_t st_;
