@@ -142,7 +142,7 @@ template <class T> __device__ __forceinline__ void vset(uint4 &v, int j, T x) {
 // rounding errors of its two products, each exact as a fused multiply-add (Dekker,
 // Numer. Math. 18, 1971), to their result: 0.51 ulp at most, 5 instructions. Below
 // 2^-33, where those errors would underflow, the cube is taken in double. Other
-// exponents take CUDA's powf. With a literal exponent only one case is compiled.
+// exponents take CUDA's powf. For exponents in the source (only one case is compiled).
 __device__ __forceinline__ float map_cube(float x) {
   const float h = x * x, r = h * x;
   const float e = __fmaf_rn(__fmaf_rn(x, x, -h), x, __fmaf_rn(h, x, -r));
@@ -431,9 +431,9 @@ MAP_PR_F1(roundf)
   __device__ __forceinline__ PR<float> pr_##fn(const PR<float> &x, const PR<float> &y) { \
     return PR<float>(fn(x.a, y.a), fn(x.b, y.b));                                       \
   }
-MAP_PR_F2(hypotf) MAP_PR_F2(fmodf) MAP_PR_F2(atan2f)
+MAP_PR_F2(powf) MAP_PR_F2(hypotf) MAP_PR_F2(fmodf) MAP_PR_F2(atan2f)
 #undef MAP_PR_F2
-__device__ __forceinline__ PR<float> pr_powf(const PR<float> &x, const PR<float> &y) {
+__device__ __forceinline__ PR<float> map_powf(const PR<float> &x, const PR<float> &y) {
   return PR<float>(map_powf(x.a, y.a), map_powf(x.b, y.b));
 }
 
