@@ -413,12 +413,11 @@ namespace {
 // Tile of a standalone Local / Focal launch. Large rasters take the tiles that move
 // the most cells per second, smaller ones flatter tiles: a wide tile's threads work
 // through 16 rows one after the other while the grid leaves SMs idle or half a wave
-// over, and the edge tiles, which do more, end last. `large`: the tile of a large
-// raster whatever g's size.
-TileCfg standalone_tile(const Group &g, bool large) {
+// over, and the edge tiles, which do more, end last.
+TileCfg standalone_tile(const Group &g) {
   TileCfg cfg;
   const FocalTune &ft = focal_tune();
-  const double cells = large ? 1e12 : (double)g.W * g.H;
+  const double cells = (double)g.W * g.H;
   if (g.skeleton == SK_FOCAL && focal_quad_form(g)) {
     // packed byte form: 128 x 16 tiles of 128 threads, a warp on the 32 words of
     // one tile row, 4 rows per thread (Life at 4096^2 with dependent launches:
@@ -431,11 +430,13 @@ TileCfg standalone_tile(const Group &g, bool large) {
     bool flow = false;
     for (Node *n : g.nodes) flow |= n->kind == K_FOCALFLOW;
     if (focal_fast_shade(g)) {
-      if ((g.H < 512 || cells > 262144) && cells < 6e6) {
+      if (cells < 6e6 && !(g.W == 512 && g.H == 512)) {
         // 64 x 16 tiles of 128 threads: 256^2 7.5 us a call against 10.3 of the 64 x 64
-        // ones (fewer than eight rows of tall tiles leave most SMs idle), 1500^2 9.8
-        // against 15.0, 2048^2 13.6 against 17.0, 3000 x 2500 under the dead border
-        // 21.5 against 21.2
+        // ones (fewer than eight rows of tall tiles leave most SMs idle), 450 x 520 7.2
+        // against 10.3, 128 x 2000 6.6 against 9.9, 1500^2 9.8 against 15.0, 2048^2 13.6
+        // against 17.0, 3000 x 2500 under the dead border 21.5 against 21.2. 512 x 512
+        // would gain too (6.5 against 10.1), but the shape test of the large tiles'
+        // kernel reads them there.
         cfg.th = 16;
       } else {
         // 64 x 64 tiles of 256 threads, 16 rows per thread (532 Gcells/s at 16384^2,
@@ -475,7 +476,7 @@ Executor::Prepared Executor::prepare(const std::vector<Node *> &targets, const s
   std::set<std::string> seen;
   for (auto &g : P.fr.groups) {
     if (g->skeleton == SK_HOST) { P.plans[g->id].skeleton = SK_HOST; continue; }
-    TileCfg cfg = standalone_tile(*g, false);
+    TileCfg cfg = standalone_tile(*g);
     P.plans[g->id] = generate_kernel(*g, cfg);
     if (compile && seen.insert(P.plans[g->id].source).second) {
       const std::string *src = &P.plans[g->id].source;
