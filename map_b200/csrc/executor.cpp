@@ -448,11 +448,15 @@ TileCfg standalone_tile(const Group &g) {
         cfg.nt = 256;
         cfg.minb = 6;
       }
-    } else if (cells < 3e6) {
-      cfg.th = 8;    // 1500^2: D8 12.1 us against 16.1 of 64 x 32, slope 11.0 against 13.7, a 3 x 3 correlation 7.9 against 11.1
-    } else if (cells < 8e6 || flow) {
-      cfg.th = 16;   // 2048^2: slope 16.3 us against 17.4, the correlation 9.8 against 11.4 (8192^2: 102 against 85); D8 8192^2 196 against 207
-    }                // else 64 x 32, 16 rows per thread
+    } else {
+      // by the cells of its tiles: flat tiles of a narrow raster are many and mostly
+      // padding (3 x 3 correlation, dead border, 64 x 8 / 64 x 16: 20 x 100000 25.1 us /
+      // 21.4, 64 x 40000 11.9 / 10.8, 200 x 14000 11.1 / 9.8; 100000 x 20 8.5 / 10.3)
+      const double tiled = (double)((g.W + 63) / 64 * 64) * g.H;
+      if (tiled < 3e6) cfg.th = 8;   // 1500^2: D8 12.1 us against 16.1 of 64 x 32, slope 11.0 against 13.7, a 3 x 3 correlation 7.9 against 11.1
+      else if (tiled < 8e6 || flow) cfg.th = 16;   // 2048^2: slope 16.3 us against 17.4, the correlation 9.8 against 11.4 (8192^2: 102 against 85); D8 8192^2 196 against 207
+      // else 64 x 32, 16 rows per thread
+    }
     if (ft.nt) cfg.nt = ft.nt;
     if (ft.tw) cfg.tw = ft.tw;
     if (ft.th) cfg.th = ft.th;
