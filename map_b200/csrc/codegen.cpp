@@ -1958,8 +1958,10 @@ static void gen_focal(Gen &G, std::ostringstream &body, std::ostringstream &wrap
            << "          }\n"
            << "        }\n";
         fx << "      }\n";
-        // out of line: few tiles run it, and the tile's own code keeps its registers
-        fix = "__device__ __noinline__ void focal_fix(const Args &a, const Tile t, unsigned char *smem) {\n" + fx.str() + "}\n";
+        // Inlined: as a call, which few tiles make, it cost the kernel 6 to 8 registers and
+        // so resident CTAs (8000^2 under the dead border, called / inlined: 5 x 5
+        // correlation 102.9 / 99.0 us, D8 198.4 / 184.5, 5 x 5 maximum 88.5 / 86.1).
+        fix = "__device__ __forceinline__ void focal_fix(const Args &a, const Tile t, unsigned char *smem) {\n" + fx.str() + "}\n";
         loop_edge += "      if (block_fixup(a.g)) focal_fix(a, t, smem);\n";
       } else {
         // the batched and serving dispatchers' persistent kernels keep the gathers: the
