@@ -38,10 +38,10 @@ long long pitch_for(int W, int dt) {
   return (b + 127) / 128 * 128;
 }
 
-// Launch phases of a batch, in stream order. A request is complete once the
-// last phase its program uses has finished.
 // CTAs that share the tiles of one request's radial scan
 constexpr long long kRadialCtas = 32;
+// Launch phases of a batch, in stream order. A request is complete once the
+// last phase its program uses has finished.
 enum Phase { PH_LEVEL0 = 0, PH_RADIAL = 1, PH_LEVEL1 = 2, PH_SPREAD = 3, N_PHASES = 4 };
 
 struct Req {
@@ -63,16 +63,23 @@ struct Req {
   std::vector<void *> scratch;
 };
 
-// How flow windows are summed: over tiles (three launches whatever the window), or,
-// by MAP_B200_SERVE_PJ, 1: pointer jumping above 64 K cells, 0: the one-CTA frontier
-// sweep (the forms of accumulations that are no 32-bit integers).
+// How a flow window is summed: over tiles (three launches whatever the window; 32-bit
+// integers whose slots' numbers fit), else by pointer jumping (integers above 64 K
+// cells) or the one-CTA frontier sweep. MAP_B200_SERVE_PJ, read once, takes the tiles
+// out: 1 leaves the jumps, 0 the sweep alone.
 enum class FlowForm { TILES, JUMP, SWEEP };
-FlowForm serve_flow() {
-  static const FlowForm v = [] {
+FlowForm flow_form(int w, int h, int dt) {
+  static const FlowForm most = [] {
     const char *e = std::getenv("MAP_B200_SERVE_PJ");
     return !e ? FlowForm::TILES : e[0] == '0' ? FlowForm::SWEEP : FlowForm::JUMP;
   }();
-  return v;
+  if (most == FlowForm::TILES && spread_tile_type(dt) && spread_tiles_fit(w, h)) return FlowForm::TILES;
+  if (most != FlowForm::SWEEP && (size_t)w * h > ((size_t)1 << 16) && spread_pj_type(dt)) return FlowForm::JUMP;
+  return FlowForm::SWEEP;
+}
+size_t flow_scratch(FlowForm f, int w, int h, int dt) {
+  const size_t N = (size_t)w * h;
+  return f == FlowForm::TILES ? spread_tile_scratch(w, h) : f == FlowForm::JUMP ? spread_pj_scratch(N, dt) : 6 * N * sizeof(int32_t);
 }
 
 size_t request_bytes(int type, int w, int h) {
@@ -94,8 +101,8 @@ struct Template {
   int last_phase = PH_LEVEL0;
 };
 
-// Flow accumulations run one CTA per request; batches take turns over several
-// streams so that consecutive batches' accumulations run side by side.
+// Batches take turns over several streams for their flow accumulations, so that
+// consecutive batches' run side by side (one CTA per request in the sweep's form).
 constexpr int kSpreadStreams = 8;
 constexpr int kQueues = 2 + kSpreadStreams;   // two batch streams, then the spreading streams
 
@@ -229,12 +236,18 @@ Template &Server::Impl::template_for(int type, int w, int h, bool compile) {
       env.kernel(P.source, P.kname + "_tiles_many", P.smem_bytes);
       T->last_phase = std::max(T->last_phase, (int)PH_RADIAL);
     } else if (g.skeleton == SK_SPREAD) {
-      env.kernel(P.source, P.kname + "_prep_many", 0);
-      env.kernel(P.source, P.kname + "_kahnp_many", 0);
-      if (spread_tile_type(P.core->meta.dtype))
-        for (const char *k : {"_flow_a_many", "_flow_b_many", "_flow_c_many"}) env.kernel(P.source, P.kname + k, 0);
-      if (spread_pj_type(P.core->meta.dtype))
-        for (const char *k : {"_pj_init_many", "_pj_step_many", "_pj_final_many"}) env.kernel(P.source, P.kname + k, 0);
+      // the kernels of the form that windows of this size take
+      switch (flow_form(w, h, P.core->meta.dtype)) {
+        case FlowForm::TILES:
+          for (const char *k : {"_flow_a_many", "_flow_b_many", "_flow_c_many"}) env.kernel(P.source, P.kname + k, 0);
+          break;
+        case FlowForm::JUMP:
+          for (const char *k : {"_pj_init_many", "_pj_step_many", "_pj_final_many"}) env.kernel(P.source, P.kname + k, 0);
+          break;
+        case FlowForm::SWEEP:
+          for (const char *k : {"_prep_many", "_kahnp_many"}) env.kernel(P.source, P.kname + k, 0);
+          break;
+      }
       T->last_phase = std::max(T->last_phase, (int)PH_SPREAD);
     } else {
       throw MapError("serving: zonal groups are not served");
@@ -381,18 +394,15 @@ void Server::Impl::run_batch(std::vector<Req *> &batch) {
           mn.tiles = std::max(mn.tiles, R.tiles);
         } else {   // SK_SPREAD
           const size_t N = (size_t)g.W * g.H;
-          const bool ft = serve_flow() == FlowForm::TILES && spread_tile_type(P.core->meta.dtype) && spread_tiles_fit(g.W, g.H);
-          const bool pj = !ft && serve_flow() != FlowForm::SWEEP && N > ((size_t)1 << 16) && spread_pj_type(P.core->meta.dtype);
+          const FlowForm form = flow_form(g.W, g.H, P.core->meta.dtype);
           // windows of one template share one launch per phase, so each form keys its own
-          Many &mn = spread[P.source + (ft ? "#tiles" : pj ? "#pj" : "")];
+          Many &mn = spread[P.source + (form == FlowForm::TILES ? "#tiles" : form == FlowForm::JUMP ? "#pj" : "")];
           mn.plan = &P;
-          mn.pj = pj;
-          if (ft) mn.tiles = std::max(mn.tiles, (long long)spread_tiles(g.W, g.H));
+          mn.pj = form == FlowForm::JUMP;
+          if (form == FlowForm::TILES) mn.tiles = std::max(mn.tiles, (long long)spread_tiles(g.W, g.H));
           mn.max_cells = std::max(mn.max_cells, N);
           void *work = nullptr;
-          const size_t wbytes = ft   ? spread_tile_scratch(g.W, g.H)
-                                : pj ? spread_pj_scratch(N, P.core->meta.dtype)
-                                     : 6 * N * sizeof(int32_t);
+          const size_t wbytes = flow_scratch(form, g.W, g.H, P.core->meta.dtype);
           cuda_check(cudaMallocAsync(&work, wbytes, st), "cudaMallocAsync(spread work)");
           r->scratch.push_back(work);
           uint64_t aux[4] = {(uint64_t)(uintptr_t)work, (uint64_t)(uintptr_t)((int32_t *)work + 2 * N),
