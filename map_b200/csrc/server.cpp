@@ -84,7 +84,8 @@ size_t flow_scratch(FlowForm f, int w, int h, int dt) {
 
 size_t request_bytes(int type, int w, int h) {
   size_t b = (size_t)pitch_for(w, F32) * h * 2;   // window copy + output
-  if (type == REQ_FLOW) b += (size_t)pitch_for(w, U8) * h + (size_t)w * h * 32;   // directions + sweep scratch
+  // directions and the accumulation's scratch (the flow program sums S32 cells)
+  if (type == REQ_FLOW) b += (size_t)pitch_for(w, U8) * h + flow_scratch(flow_form(w, h, S32), w, h, S32);
   return b;
 }
 

@@ -1,11 +1,16 @@
-"""Flow accumulations in serving: the forms that stand in for the tiles
-(MAP_B200_SERVE_PJ: pointer jumping above 64 K cells, the one-CTA sweep below or alone) give the same cells. The variable
+"""Flow accumulations in serving: the memory a request is charged is what its form
+takes, and the forms that stand in for the tiles (MAP_B200_SERVE_PJ: pointer jumping
+above 64 K cells, the one-CTA sweep below or alone) give the same cells. The variable
 is read once, so each form runs in a process of its own."""
+import ctypes as ct
 import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
+
+from map_b200 import synth
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +43,22 @@ def test_forms_agree(form):
         env["MAP_B200_SERVE_PJ"] = form
     r = subprocess.run([sys.executable, "-c", PROGRAM], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip().endswith("same"), r.stderr[-2000:]
+
+
+def test_charged_what_the_tiles_take(M):
+    # two 512 x 512 flow windows: rasters and directions 2.3 MB each, the tiles' scratch 0.3 MB
+    dem = synth.fbm_dem(600, 600, seed=5)
+    d = M._lib.ma_devAlloc(dem.nbytes)
+    M._lib.ma_memcpy(ct.c_void_p(d), dem.ctypes.data_as(ct.c_void_p), dem.nbytes, 1)
+    budget = 6 << 20
+    srv = M.Server(d, 600 * 4, 600, 600, budget_bytes=budget, max_batch=8)
+    try:
+        ids = [srv.submit(M.Server.FLOW, 8 * k, 4 * k, 512, 512) for k in range(5)]
+        outs = [srv.result(i, (512, 512), np.int32) for i in ids]
+        st = srv.stats()
+        assert st["completed"] == 5 and 2 * 512 * 512 * 4 < st["peak_bytes"] <= budget
+        win = M.from_numpy(np.ascontiguousarray(dem[8:520, 16:528]), bs=[512, 512])
+        assert np.array_equal(outs[2], M.to_numpy(M.flow_accumulation(M.ones_like(win, M.S32), M.flow_direction(win))))
+    finally:
+        srv.close()
+        M._lib.ma_devFree(ct.c_void_p(d))
