@@ -30,4 +30,4 @@ def test_both_callers_ask():
     for name, calls in (("codegen_scan.cpp", 1), ("server.cpp", 1)):
         text = open(os.path.join(CSRC, name)).read()
         assert text.count("spread_tile_type(") - text.count("bool spread_tile_type(") >= calls
-        assert "spread_tiles_fit(g.W, g.H)" in text
+        assert "spread_tiles_fit(" in text
