@@ -1589,7 +1589,7 @@ static void gen_focal(Gen &G, std::ostringstream &body, std::ostringstream &wrap
   // (by default for the fast hillshade form, whose interior tiles keep their
   // results in registers one cell per thread step, the form the store serves)
   const FocalTune &ft0 = focal_tune();
-  if (P.tile_store && nst > 0 && G.outk.size() == 1 &&
+  if (P.standalone && nst > 0 && G.outk.size() == 1 &&
       (ft0.tstore >= 2 || (ft0.tstore == 1 && G.any_fast() && !ft0.fpair && !ft0.cpair))) {
     Node *o = G.outk.begin()->first;
     const int es = (int)dt_size(o->meta.dtype);
@@ -1879,11 +1879,11 @@ static void gen_focal(Gen &G, std::ostringstream &body, std::ostringstream &wrap
     int align_e = 1;
     for (auto &t : P.tma) align_e = std::max(align_e, 16 / (int)dt_size(t.dtype));
     body << "  const bool inner = tile_interior<" << TW << ", " << TH << ">(a.g, t, " << hx << ", " << hy << ");\n"
-         << "  if (t.x0 % " << align_e << " == 0" << (P.tile_store ? " || a.aux[3] != 0" : "") << ") {\n"
+         << "  if (t.x0 % " << align_e << " == 0" << (P.standalone ? " || a.aux[3] != 0" : "") << ") {\n"
          << "    if (gdesc) __syncthreads();   // a persistent CTA: earlier readers of the staging buffer are done\n";
     // aux[3]: an input whose rows start on no 16-byte boundary has no tensor map (the
     // executor's own launches; the batched and serving dispatchers align their inputs)
-    if (P.tile_store) {
+    if (P.standalone) {
       body << "    if (a.aux[3] != 0) {\n";
       for (int k = 0; k < nst; k++) {
         auto &t = P.tma[k];
@@ -1910,7 +1910,7 @@ static void gen_focal(Gen &G, std::ostringstream &body, std::ostringstream &wrap
          << "      return false;\n"
          << "    }\n"
          << "    phase ^= 1u;\n"
-         << (P.tile_store ? "    }\n" : "") << "    if (!inner) {\n";
+         << (P.standalone ? "    }\n" : "") << "    if (!inner) {\n";
     for (int k = 0; k < nst; k++) {
       auto &t = P.tma[k];
       std::string ty = dt_ctype(t.dtype);
@@ -1930,7 +1930,7 @@ static void gen_focal(Gen &G, std::ostringstream &body, std::ostringstream &wrap
     // threads (after their own stores of the same cells)
     {
       std::ostringstream fx;
-      if (P.tile_store) {
+      if (P.standalone) {
         fx << "      {\n";
         std::string taps, call1 = "focal_cell(a";
         for (int k = 0; k < nst; k++) {
@@ -2169,24 +2169,16 @@ static std::string gen_zonal(Gen &G) {
   return s.str();
 }
 
-// Radiating skeleton (runtime/skeleton/RadiatingSkeleton.cpp:32-323): one CTA per
-// octant sweeps the fronts d0 = 1, 2, ... in order; a front's cells are spread over
-// the CTA's threads. A cell's scan value is op(LIT(front d0-1 at d1, at d1-1), in)
-// when `in` is finite; the start cell holds the neutral value. The previous front
-// is read back (L1-bypassing loads) from the scan's own output raster, written by
-// this CTA one step earlier; cells on an octant boundary are written by both
-// adjacent octants with identical values. Local nodes before the scan produce
-// `in` per cell; those after it run right after the cell's scan value.
 // The tiled form of a radial scan: an octant's triangle of (front, cell) pairs is
 // cut into strips of RADIAL_T fronts and tiles of RADIAL_B cells. A tile is one CTA's
 // work item:
-//   1. all threads evaluate the scan's argument and the interpolation weight of
-//      the tile's cells (and of the RADIAL_T cells left of it that its own cells
-//      depend on: a cell reads the previous front at d1 and d1 - 1) into shared
-//      memory, along x whichever way the octant runs;
+//   1. all threads evaluate the scan's argument of the tile's cells (and of the
+//      RADIAL_T cells left of it that its own cells depend on: a cell reads the
+//      previous front at d1 and d1 - 1) into shared memory, along x whichever way
+//      the octant runs;
 //   2. warp 0 takes the last front of the previous strip from the scratch area,
-//      sweeps the strip's fronts in registers, neighbours by shuffles, no
-//      barrier between fronts, and publishes its last front;
+//      sweeps the strip's fronts in registers with their interpolation weights,
+//      neighbours by shuffles, no barrier between fronts, and publishes its last front;
 //   3. all threads evaluate the nodes after the scan and store the outputs.
 // Tiles are claimed by ticket in strip order, so the tiles a claimed tile waits
 // for are held by CTAs already running: the wait (bounded) needs no co-residency
@@ -2197,7 +2189,7 @@ static std::string radial_tiles_source(Gen &G, const std::string &T) {
   KernelPlan &P = G.plan;
   Node *scan = P.core;
   const std::string v = G.val(scan);
-  const std::string arg = G.val(scan->prev[0]), AT = G.T(scan->prev[0]);
+  const std::string arg = G.val(scan->prev[0]);
   P.smem_bytes = radial_tile_smem(scan->meta.dtype);
   std::ostringstream s;
   // the scan's argument at one cell, and the nodes after the scan
@@ -2243,6 +2235,15 @@ static std::string radial_tiles_source(Gen &G, const std::string &T) {
   return s.str();
 }
 
+// Radiating skeleton (runtime/skeleton/RadiatingSkeleton.cpp:32-323): the tiled form
+// above, and the forms without scratch memory: one CTA per octant (or a cluster) sweeps
+// the fronts d0 = 1, 2, ... in order; a front's cells are spread over the CTA's threads.
+// A cell's scan value is op(LIT(front d0-1 at d1, at d1-1), in)
+// when `in` is finite; the start cell holds the neutral value. The previous front
+// is read back (L1-bypassing loads) from the scan's own output raster, written by
+// this CTA one step earlier; cells on an octant boundary are written by both
+// adjacent octants with identical values. Local nodes before the scan produce
+// `in` per cell; those after it run right after the cell's scan value.
 static std::string gen_radial(Gen &G) {
   KernelPlan &P = G.plan;
   Node *scan = P.core;
@@ -3024,7 +3025,7 @@ KernelPlan generate_kernel(const Group &g, TileCfg cfg) {
   P.tile_w = cfg.tw;
   P.tile_h = cfg.th;
   P.min_blocks = cfg.minb;
-  P.tile_store = cfg.tile_store;
+  P.standalone = cfg.standalone;
   Gen G(g, P);
   G.classify();
   std::string src;
