@@ -2840,11 +2840,11 @@ static std::string gen_spread(Gen &G) {
       << "  return (a.g.W + FLOW_T - 1) / FLOW_T * ((a.g.H + FLOW_T - 1) / FLOW_T);\n"
       << "}\n";
     for (int fin = 0; fin < 2; fin++)
-      s << "extern \"C\" __global__ void __launch_bounds__(FLOW_NT) KNAME_flow_" << (fin ? "c" : "a")
+      s << "extern \"C\" __global__ void __launch_bounds__(FLOW_NT, 5) KNAME_flow_" << (fin ? "c" : "a")
         << "(const __grid_constant__ Args a) {\n"
         << "  flow_tile<FlowOps, " << (fin ? "true" : "false") << ">(a, a.in[" << kd << "], a.out[" << ko << "], (int)blockIdx.x);\n"
         << "}\n"
-        << "extern \"C\" __global__ void __launch_bounds__(FLOW_NT) KNAME_flow_" << (fin ? "c" : "a")
+        << "extern \"C\" __global__ void __launch_bounds__(FLOW_NT, 5) KNAME_flow_" << (fin ? "c" : "a")
         << "_many(const __grid_constant__ FlowManyArgs m) {\n"
         << "  const s64 r = blockIdx.x / m.per;\n"
         << "  if (r >= m.n) return;\n"

@@ -887,10 +887,11 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
       // straight into the caller's buffer, where that may be written in place; rows on
       // no 16-byte boundary only where no other group reads the raster back
       const long long es = (long long)dt_size(o->meta.dtype);
-      const bool aligned = ((uintptr_t)s->dev & 127) == 0 && (s->dev_pitch & 15) == 0 && in_place(o, *s);
-      const bool apart = (uintptr_t)s->dev % (uintptr_t)es == 0 && s->dev_pitch % es == 0 && readers(o) == 0 && !in_chain(o) &&
-                         !meets_input(*s);
-      if ((aligned || apart) && s->dev_pitch >= (long long)o->meta.W() * es) {
+      const bool aligned = ((uintptr_t)s->dev & 127) == 0 && (s->dev_pitch & 15) == 0;
+      const bool there = aligned ? in_place(o, *s)
+                                 : (uintptr_t)s->dev % (uintptr_t)es == 0 && s->dev_pitch % es == 0 && readers(o) == 0 &&
+                                       !in_chain(o) && !meets_input(*s);
+      if (there && s->dev_pitch >= (long long)o->meta.W() * es) {
         DevRaster r;
         r.ptr = s->dev;
         r.pitch = s->dev_pitch;

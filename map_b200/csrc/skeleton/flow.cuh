@@ -16,9 +16,10 @@
 //
 // 2048^2 (fBm, 4.2 M cells): 42 + 7 + 38 us for the passes, against 46 + 540 us for
 // counting and walking the whole raster, whose longest path of one L2 atomic per cell
-// bounds it. The tiles' passes are bound by shared-memory latency at four CTAs per SM
-// (62 registers; five or six measured the same). Tried for the tiles: walks with
-// counts 200 us a pass (a thread's longest walk sets the tile's time), doubling in
+// bounds it. The tiles' passes are bound by shared-memory latency at five CTAs per SM
+// (launch bounds; passes on terrain of 2048^2 / 3000^2: four 78.7 / 97.1 us, five 76.3 /
+// 91.0, six 76.6 / 90.4 and random codes slower, none given 78.7 / 94.0). Tried for the
+// tiles: walks with counts 200 us a pass (a thread's longest walk sets the tile's time), doubling in
 // pass C too 56 us. Random codes, full of cycles, at 2048^2: 124 us, against 279 of the
 // whole-raster walks and 642 when tiles with a cycle took walks with counts.
 #pragma once
@@ -249,12 +250,17 @@ __device__ __forceinline__ void flow_tile(const ARGS &a, const RasterArg &D, con
       }
     }
     __syncthreads();
+    // (the cycles' cells, which hold no other tile's water, first: zero)
+    if (cycles) {
+      for (int k = 0; k < PER; ++k) {
+        const int i = tid + k * FLOW_NT, cx = i % FLOW_T, cy = i / FLOW_T;
+        if (cx < w && cy < h && marked(i)) sum[i] = OPS::water(a, x0 + cx, y0 + cy);
+      }
+    }
 #pragma unroll 4
     for (int k = 0; k < PER; ++k) {
       const int i = tid + k * FLOW_NT, cx = i % FLOW_T, cy = i / FLOW_T;
-      if (cx >= w || cy >= h) continue;
-      const bool whole = !cycles || !marked(i);
-      *cell_ptr<u32>(O, x0 + cx, y0 + cy) = whole ? sum[i] - OPS::water(a, x0 + cx, y0 + cy) : 0u;
+      if (cx < w && cy < h) *cell_ptr<u32>(O, x0 + cx, y0 + cy) = sum[i] - OPS::water(a, x0 + cx, y0 + cy);
     }
   }
 }
