@@ -564,8 +564,10 @@ std::shared_ptr<Executor::Prepared> Executor::prepare_cached(const std::vector<N
   }
   for (Node *t : targets)
     if (t->meta.numdim != D0) P->need_device = true;
-  for (Node *n : P->order)
+  for (Node *n : P->order) {
     if (n->meta.numdim == D0) P->d0.push_back(n);
+    if (n->kind == K_DEVIN) P->dev_in.push_back(n);
+  }
   if (cache_.size() >= 64) {   // evict the least recently used entry
     auto lru = cache_.begin();
     for (auto c = cache_.begin(); c != cache_.end(); ++c)
@@ -808,8 +810,8 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
     return false;
   };
   auto meets_input = [&](const Sink &s) {
-    for (Node *n : P.order)
-      if (n->kind == K_DEVIN && meets(n->dev->ptr, n->dev->pitch, n->meta.H(), s.dev, s.dev_pitch, s.node->meta.H())) return true;
+    for (Node *n : P.dev_in)
+      if (meets(n->dev->ptr, n->dev->pitch, n->meta.H(), s.dev, s.dev_pitch, s.node->meta.H())) return true;
     return false;
   };
   // groups that read raster n (a chain's first group counts as several: its tiles
@@ -874,8 +876,8 @@ void Executor::evaluate(const std::vector<Node *> &targets_in, const std::vector
     return false;
   };
   auto in_place = [&](Node *o, const Sink &s) {
-    for (Node *n : P.order)
-      if (n->kind == K_DEVIN && meets(n->dev->ptr, n->dev->pitch, n->meta.H(), s.dev, s.dev_pitch, s.node->meta.H()) &&
+    for (Node *n : P.dev_in)
+      if (meets(n->dev->ptr, n->dev->pitch, n->meta.H(), s.dev, s.dev_pitch, s.node->meta.H()) &&
           !writable_over(P.fr, P.plans, o, n, n->dev->ptr == s.dev && n->dev->pitch == s.dev_pitch, rt.exec_mode == EXEC_FUSED))
         return false;
     return true;

@@ -131,6 +131,7 @@ class Executor {
     bool foldable = false;       // some group's outputs may all be fixed (predict_group is worth a look)
     bool need_device = false;    // some group runs on the device
     std::vector<Node *> d0;      // the scalar nodes of `order`
+    std::vector<Node *> dev_in;  // its device inputs
   };
   Prepared prepare(const std::vector<Node *> &targets, const std::set<Node *> &tset, bool compile);
   static void find_chains(Prepared &P, const std::set<Node *> &tset);
