@@ -196,7 +196,8 @@ ma_Node *ma_fromDevice(void *dptr, long long pitch, ma_Array ds, int dt, ma_Arra
  *   ds raster, `dptr` the address of row row0 (16-byte aligned, pitch a
  *   multiple of 16 bytes). Such an input is evaluated by ma_evalRows only.
  * ma_evalRows: evaluates rows [y0, y1) of the n rasters into device memory
- *   dst[i] (the address of row y0, pitch[i] bytes between rows). The program
+ *   dst[i] (the address of row y0, pitch[i] bytes between rows; may lie in an
+ *   input's rows). The program
  *   must consist of Local and Focal groups over one raster shape, with device
  *   inputs holding at least rows [y0 - m, y1 + m) (clipped to the raster),
  *   m = ma_rowMargin(...). Border rules are applied in whole-raster
@@ -222,7 +223,9 @@ int ma_binWriteHost(const char *path, const void *src, ma_Array ds, int dt, int 
 /* Evaluate `node` and copy the raster to dense row-major host memory of
  * `bytes` bytes. Returns 0 on success. */
 int ma_toHost(ma_Node *node, void *dst, size_t bytes);
-/* Evaluate `node` into device memory (written in place when possible).
+/* Evaluate `node` into device memory, written directly when possible; dptr may lie
+ * in the memory of device inputs (the result then goes through a buffer unless the
+ * program is element-wise).
  * With async != 0 the call returns once the work is enqueued on the library's
  * stream (see ma_stream / ma_sync). Returns 0 on success. */
 int ma_toDevice(ma_Node *node, void *dptr, long long pitch, int async);
@@ -251,7 +254,7 @@ int ma_memcpy(void *dst, const void *src, size_t bytes, int kind); /* kind as cu
  * driven by a device work-list of (kernel kind, instance, tile) items and
  * replayed from a CUDA graph. Only Local and Focal groups can be batched; inputs
  * must be device-resident, host or file rasters; outputs go to caller device
- * buffers (16-byte aligned base and pitch).
+ * buffers (16-byte aligned base and pitch) that share no memory with an input.
  * ma_batchAdd returns the instance index; ma_batchPrepare fuses, autotunes tile
  * shapes (autotune != 0), compiles and captures the graph (called by the first
  * ma_batchRun when omitted); ma_batchInfo writes a JSON description.
